@@ -741,42 +741,6 @@ size_t xw_smem() {
   return sizeof(CX) * (NX + XW_WARPS * MAXP * padded_len(NX) + XW_WARPS * (5 + NTH) * (NX / 3 + 1));
 }
 
-// Planes one x-row CTA marches through when the tuning leaves it automatic
-// (DG_TUNE_XROW_CHUNK = 0): the fewest (at least 3) that fit the whole grid
-// into one wave of resident CTAs, so no SM waits out a partial last wave;
-// grids too large for that take 32 planes per CTA.
-int xrow_auto_chunk(int nplan, int NZ, const void *kern, size_t smem) {
-  static std::mutex mu;
-  static std::map<std::pair<const void *, size_t>, int> per_sm_cache;
-  static int nsm = 0;
-  int per_sm = 0;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (!nsm) {
-      int dev = 0;
-      cudaGetDevice(&dev);
-      if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        nsm = 148;
-    }
-    auto it = per_sm_cache.find({kern, smem});
-    if (it != per_sm_cache.end()) {
-      per_sm = it->second;
-    } else {
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * XW_WARPS, smem) !=
-          cudaSuccess)
-        per_sm = 1;
-      per_sm_cache[{kern, smem}] = per_sm;
-    }
-  }
-  const long slots = (long)(per_sm > 0 ? per_sm : 1) * nsm;
-  const long zb = dg_cdiv(NZ, XW_WARPS);
-  const long per_col = slots / zb > 0 ? slots / zb : 1;  // CTAs per z-block column in one wave
-  int chunk = dg_cdiv(nplan, per_col);
-  if (chunk < 3) chunk = 3;
-  if (chunk > 32) chunk = 32;
-  return chunk < nplan ? chunk : nplan;
-}
-
 // the plan variant of the handle's tuning, for lengths that have one
 template <int NX, int NTH, typename CX>
 auto xrow_kernel(int v) {
@@ -1796,6 +1760,52 @@ __global__ void k_absmax(const double *__restrict__ a, long n, unsigned long lon
 }  // namespace
 
 // ================================================================ host side
+// Planes one CTA of a marching kernel takes (k_xrow_w, k_xmarch) when the
+// tuning leaves it automatic (DG_TUNE_XROW_CHUNK = 0).  A CTA costs `per`
+// for each of its planes and `lead` for the planes it loads before the first
+// one; the chunk is the one whose waves of resident CTAs cost least in all.
+// On a small grid that spreads the planes over the idle SMs (one plane per
+// CTA if they fit one wave), on a large one it keeps the chunks long and the
+// last wave full.
+int dg_march_chunk(int nplan, int rows, const void *kern, int threads, size_t smem, double per,
+                   double lead) {
+  static std::mutex mu;
+  static std::map<std::pair<const void *, size_t>, int> per_sm_cache;
+  static int nsm = 0;
+  int per_sm = 0;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!nsm) {
+      int dev = 0;
+      cudaGetDevice(&dev);
+      if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        nsm = 148;
+    }
+    auto it = per_sm_cache.find({kern, smem});
+    if (it != per_sm_cache.end()) {
+      per_sm = it->second;
+    } else {
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) !=
+          cudaSuccess)
+        per_sm = 1;
+      per_sm_cache[{kern, smem}] = per_sm;
+    }
+  }
+  const long slots = (long)(per_sm > 0 ? per_sm : 1) * nsm;
+  int best = nplan;
+  double cost = 1e300;
+  for (int n = 1; n <= nplan; n++) {
+    const int c = dg_cdiv(nplan, n);
+    const long ctas = (long)rows * dg_cdiv(nplan, c);
+    const double v = (double)((ctas + slots - 1) / slots) * (per * c + lead);
+    if (v < cost) {
+      cost = v;
+      best = c;
+    }
+  }
+  return best;
+}
+
 // Row templates of the CN systems (host, once per handle).
 static void cn_row_templates(const dg_handle *h, double *rows) {
   const int NY = h->NY, L = NY + 2, nfld = h->nf;
@@ -2060,8 +2070,9 @@ static int nl_chunk_mixed(dg_handle *h, const ChanConst &C, int rk_step, int a, 
     auto kern = xrow_kernel<NXV, NTHV, float2>(h->fft_plan);                                    \
     dg_big_smem((const void *)kern);                                                            \
     int chunk = h->xrow_chunk > 0 ? (h->xrow_chunk < nplan ? h->xrow_chunk : nplan)            \
-                                  : xrow_auto_chunk(nplan, h->NZ, (const void *)kern,          \
-                                                    xw_smem<NXV, NTHV, float2>());              \
+                                  : dg_march_chunk(nplan, dg_cdiv(h->NZ, XW_WARPS),             \
+                                                   (const void *)kern, 32 * XW_WARPS,           \
+                                                   xw_smem<NXV, NTHV, float2>(), 1.0, 1.0);     \
     dim3 grid(dg_cdiv(h->NZ, XW_WARPS), dg_cdiv(nplan, chunk));                                 \
     dg_kt_begin(h, "k_xrow_w_f32", h->st);                                                      \
     DG_CUDA(dg_launch(h->pdl, kern, grid, dim3(32 * XW_WARPS),                                  \
@@ -2117,47 +2128,51 @@ static int nl_generic_mixed(dg_handle *h, const ChanConst &C, int rk_step,
                             Hf, Hfield);
   h->pdl_zinv = 0;
   DG_TRY(zs);
-  // work: FP32 fluctuation rows [nf][NY+2][NZ][NX], then FP64 row means [nf][NY+2][NZ]
-  const long pplane = (long)NZ * NX, pfield = (long)(NY + 2) * pplane;
-  float *phys = reinterpret_cast<float *>(h->work);
-  double *dc = reinterpret_cast<double *>(phys + h->nf * pfield);
-  const long dfield = (long)(NY + 2) * NZ;
   bool done = false;
-  {
-    dim3 grid(dg_cdiv(NZ, 8), NY + 2, h->nf);
-    const size_t sm = sizeof(float2) * (NX + 4 * (size_t)padded_len(NX));
+  if (dg_xmarch_ok(h)) {
+    DG_TRY(dg_xmarch(h));
+  } else {
+    // work: FP32 fluctuation rows [nf][NY+2][NZ][NX], then FP64 row means [nf][NY+2][NZ]
+    const long pplane = (long)NZ * NX, pfield = (long)(NY + 2) * pplane;
+    float *phys = reinterpret_cast<float *>(h->work);
+    double *dc = reinterpret_cast<double *>(phys + h->nf * pfield);
+    const long dfield = (long)(NY + 2) * NZ;
+    {
+      dim3 grid(dg_cdiv(NZ, 8), NY + 2, h->nf);
+      const size_t sm = sizeof(float2) * (NX + 4 * (size_t)padded_len(NX));
 #define XC_CASE(N)                                                                              \
-  if (!done && NX == N) {                                                                       \
-    dg_big_smem((const void *)k_xc2r_f<N>);                                                     \
-    dg_kt_begin(h, "k_xc2r_f32", h->st);                                                        \
-    DG_CUDA(dg_launch(h->pdl, k_xc2r_f<N>, grid, dim3(128), sm, h->st, Hf, Hfield, NZ, h->nkxp, \
-                      h->twx_f, phys, pfield, dc, dfield));                                     \
-    done = true;                                                                                \
-  }
-    DG_FOR_EACH_N(XC_CASE)
+    if (!done && NX == N) {                                                                       \
+      dg_big_smem((const void *)k_xc2r_f<N>);                                                     \
+      dg_kt_begin(h, "k_xc2r_f32", h->st);                                                        \
+      DG_CUDA(dg_launch(h->pdl, k_xc2r_f<N>, grid, dim3(128), sm, h->st, Hf, Hfield, NZ, h->nkxp, \
+                        h->twx_f, phys, pfield, dc, dfield));                                     \
+      done = true;                                                                                \
+    }
+      DG_FOR_EACH_N(XC_CASE)
 #undef XC_CASE
-  }
-  if (!done) {
-    dg_set_error("mixed precision: no FP32 x-row kernel for this NX");
-    return DG_ERR_DIMS;
-  }
-  DG_LAUNCHED();
-  done = false;
-  {
-    dim3 grid(xp_pairs(h->NTH), dg_cdiv(NZ, XP_THR / 32), NY);
-    const size_t sm = sizeof(float2) * (NX + (XP_THR / 32) * (size_t)padded_len(NX));
+    }
+    if (!done) {
+      dg_set_error("mixed precision: no FP32 x-row kernel for this NX");
+      return DG_ERR_DIMS;
+    }
+    DG_LAUNCHED();
+    done = false;
+    {
+      dim3 grid(xp_pairs(h->NTH), dg_cdiv(NZ, XP_THR / 32), NY);
+      const size_t sm = sizeof(float2) * (NX + (XP_THR / 32) * (size_t)padded_len(NX));
 #define XP_CASE(N)                                                                              \
-  if (!done && NX == N) {                                                                       \
-    dg_big_smem((const void *)k_xprod_f<N>);                                                    \
-    dg_kt_begin(h, "k_xprod_f32", h->st);                                                       \
-    DG_CUDA(dg_launch(h->pdl, k_xprod_f<N>, grid, dim3(XP_THR), sm, h->st, C, phys, pfield, dc, \
-                      dfield, h->twx_f, h->dyf, h->dy, h->kx, Gf, Hfield));                     \
-    done = true;                                                                                \
-  }
-    DG_FOR_EACH_N(XP_CASE)
+    if (!done && NX == N) {                                                                       \
+      dg_big_smem((const void *)k_xprod_f<N>);                                                    \
+      dg_kt_begin(h, "k_xprod_f32", h->st);                                                       \
+      DG_CUDA(dg_launch(h->pdl, k_xprod_f<N>, grid, dim3(XP_THR), sm, h->st, C, phys, pfield, dc, \
+                        dfield, h->twx_f, h->dyf, h->dy, h->kx, Gf, Hfield));                     \
+      done = true;                                                                                \
+    }
+      DG_FOR_EACH_N(XP_CASE)
 #undef XP_CASE
+    }
+    DG_LAUNCHED();
   }
-  DG_LAUNCHED();
   done = false;
   dim3 zgrid(dg_cdiv(h->nkxp, zw_kxg(NZ)), NY, h->nf);
   const size_t sm = zw_smem<float2>(NZ);
@@ -2238,8 +2253,9 @@ int dg_chan_nonlinear(dg_handle *h, int time_step, int rk_step, bool *column_nex
     auto kern = xrow_kernel<NXV, NTHV, double2>(h->fft_plan);                                    \
     dg_big_smem((const void *)kern);                                                             \
     int chunk = h->xrow_chunk > 0 ? (h->xrow_chunk < nplan ? h->xrow_chunk : nplan)             \
-                                  : xrow_auto_chunk(nplan, h->NZ, (const void *)kern,           \
-                                                    xw_smem<NXV, NTHV>());                       \
+                                  : dg_march_chunk(nplan, dg_cdiv(h->NZ, XW_WARPS),             \
+                                                   (const void *)kern, 32 * XW_WARPS,           \
+                                                   xw_smem<NXV, NTHV>(), 1.0, 1.0);             \
     dim3 grid(dg_cdiv(h->NZ, XW_WARPS), dg_cdiv(nplan, chunk));                                  \
     dg_kt_begin(h, "k_xrow_w", h->st);                                                             \
     DG_CUDA(dg_launch(h->pdl, kern, grid, dim3(32 * XW_WARPS),                                   \
@@ -2258,25 +2274,29 @@ int dg_chan_nonlinear(dg_handle *h, int time_step, int rk_step, bool *column_nex
       if (a == 1) {
         DG_TRY(dg_zinv(h, in, h->nf, hdone + 1, h->NY + 1, h->H, 0));
         hdone = h->NY + 1;
-        // every plane to physical space (the work array holds nf stacks of
-        // NY+2 planes), then the products of planes 1..NY
-        const long pplane = (long)h->NZ * h->NX, pfield = (long)(h->NY + 2) * pplane;
-        double *phys = (double *)h->work;
-        DG_TRY(dg_xc2r_planes(h, h->H, h->nf, 0, h->NY + 1, phys, pplane, h->NX, pfield));
-        const int rz = xp_rows(h->NX);
-        dim3 grid(xp_pairs(h->NTH), dg_cdiv(h->NZ, rz), h->NY);
-        const size_t sm = xp_smem(h->NX, rz);
+        if (dg_xmarch_ok(h)) {
+          DG_TRY(dg_xmarch(h));
+        } else {
+          // every plane to physical space (the work array holds nf stacks of
+          // NY+2 planes), then the products of planes 1..NY
+          const long pplane = (long)h->NZ * h->NX, pfield = (long)(h->NY + 2) * pplane;
+          double *phys = (double *)h->work;
+          DG_TRY(dg_xc2r_planes(h, h->H, h->nf, 0, h->NY + 1, phys, pplane, h->NX, pfield));
+          const int rz = xp_rows(h->NX);
+          dim3 grid(xp_pairs(h->NTH), dg_cdiv(h->NZ, rz), h->NY);
+          const size_t sm = xp_smem(h->NX, rz);
 #define KERNEL_BODY(N)                                                                          \
-  dg_big_smem((const void *)k_xprod<N>);                                                        \
-  dg_kt_begin(h, "k_xprod", h->st);                                                             \
-  k_xprod<N><<<grid, XP_THR, sm, h->st>>>(C, phys, pfield, rz, h->plx, h->twx, h->dyf, h->dy,   \
-                                          h->kx, h->G, Hfield)
-        switch (h->NX) {
-          DG_FOR_EACH_N(DG_CASE_N)
-          default: KERNEL_BODY(0); break;
-        }
+    dg_big_smem((const void *)k_xprod<N>);                                                        \
+    dg_kt_begin(h, "k_xprod", h->st);                                                             \
+    k_xprod<N><<<grid, XP_THR, sm, h->st>>>(C, phys, pfield, rz, h->plx, h->twx, h->dyf, h->dy,   \
+                                            h->kx, h->G, Hfield)
+          switch (h->NX) {
+            DG_FOR_EACH_N(DG_CASE_N)
+            default: KERNEL_BODY(0); break;
+          }
 #undef KERNEL_BODY
-        DG_LAUNCHED();
+          DG_LAUNCHED();
+        }
       }
     }
     // 3. z forward, explicit terms, CN right-hand side for planes a..b (all

@@ -233,6 +233,10 @@ int dg_plane_r2c(dg_handle *h, const double *phys, int nf, int jmin, int jmax,
 int dg_chan_init(dg_handle *h);
 int dg_per_init(dg_handle *h);
 int dg_apply_bc_vel_dev(dg_handle *h);
+int dg_march_chunk(int nplan, int rows, const void *kern, int threads, size_t smem, double per,
+                   double lead);
+bool dg_xmarch_ok(const dg_handle *h);  // the x-row stage runs as k_xmarch
+int dg_xmarch(dg_handle *h);
 int dg_rem_div_dev(dg_handle *h, int update_cp, int rk_step, bool from_rhs);
 int dg_courant_dev(dg_handle *h, const double2 *const *u, bool side = false);
 int dg_stats_dev(dg_handle *h, dg_stats *s);
