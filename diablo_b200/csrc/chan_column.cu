@@ -12,33 +12,39 @@
 //   CN solves        for/channel.f:771-1029 (THOMAS_*_MPI, for/mpi.f:630-866)
 // REM_DIV_CHAN and the pressure update follow as their own launch (k_rd_col).
 //
-// A work item is (case, mode tile, field); one thread per (mode, segment of
-// SEG_K consecutive rows).  The CN system of a field is the same for every
+// A work item is (case, mode tile, field), one CTA; one thread per (mode,
+// segment of K consecutive rows), the modes of a segment in neighbouring
+// lanes.  The CN system of a field is the same for every
 // mode, and its elimination (the substep's table: multipliers a, reciprocal
 // pivots 1/b, f = -c/b) turns the solve into two first-order linear
 // recurrences, forward g(j) = r(j) + a(j) g(j-1) and backward
 // x(j) = e(j) + f(j) x(j+1) with e = g/b.  A linear recurrence splits exactly
 // over segments: each thread runs its segment from a zero start, keeping the
-// product of the coefficients; one lane per mode then carries the segment
-// ends across the column (one step per segment instead of one per row), and
-// each thread adds carry x product to its rows.  The same algebra as
-// THOMAS_FORWARD / THOMAS_BACKWARD, with the rounding of a different order
-// of the same operations.  Segment boundaries depend only on NY, so a mode's
-// arithmetic does not depend on the tile width.
+// product of the coefficients; the (product, end value) of the segments, four at a time
+// by shuffles and then quad by quad from shared memory, carry the
+// segment ends through the column, and each thread adds carry x product to its rows.  The same
+// algebra as THOMAS_FORWARD / THOMAS_BACKWARD, with the rounding of a different
+// order of the same operations.  Segments and quads depend only on NY, so a
+// mode's arithmetic does not depend on the tile width.
 //
-// One CTA per work item.  One thread fetches the field's CU tile and the NL
-// term the z-forward kernel left in the field's rhs array by bulk tensor
-// copies (TMA, no multicast), and the table and grid-factor rows by bulk
-// copies, all at once on one mbarrier with a bounded wait.  The right-hand
-// side is formed in a flat loop over (row, mode) -- CF_old and CP read there
-// in batches, each batch's loads issued before its stores -- and replaces
-// NL in shared memory,
-// the recurrences run there (each phase loads its rows before its chain),
-// and the post-CN field goes to the field's rhs array.  CU is read-only in
-// this kernel, so a field's right-hand side may read another field
-// (rotation, buoyancy, GRAV, DRHODX/Z) without a race.  REM_DIV then reads
-// the post-CN velocity from the rhs arrays and writes CU.  A scalar that no
-// velocity right-hand side reads is written in place.
+// Everything between the inputs and the post-CN field is in the thread's
+// registers: it loads its rows of CU, NL (which the z-forward kernel left in the
+// field's rhs array), CF_old and CP straight from global memory -- the lanes of a segment
+// read neighbouring modes, whole sectors -- forms R, runs the recurrences and stores CF and the
+// field, with one barrier per direction for the quads' totals.  Only the table
+// and grid-factor rows, shared by every mode, go through shared memory (bulk
+// copies on one mbarrier with a bounded wait).  CU is read-only in this kernel,
+// so a field's right-hand side may read another field (rotation, buoyancy, GRAV,
+// DRHODX/Z) without a race.  REM_DIV then reads the post-CN velocity from the rhs
+// arrays and writes CU.  A scalar that no velocity right-hand side reads is
+// written in place.
+//
+// It is bound by memory latency: 114 MB per launch at Re_tau = 180 in 41 us (1107 us
+// at 512x257x384 with a scalar), 14 warps per SM at 128 registers.  Forms with the columns in shared memory (bulk
+// tensor copies of CU and NL, CF and CP read beside them, the recurrences there with six
+// barriers) took 52 us at 4 modes per CTA and 43 at 8 (1302 and 1042), and 51 with all four tiles staged and the
+// recurrences in registers: the tiles allow two to four CTAs per SM, and each
+// waits for its copies, computes and writes in turn.
 //
 // The same kernel serves one case (a one-case table) and the ensemble
 // server's groups (a ragged work list over every member), so a case
@@ -52,11 +58,12 @@
 
 namespace {
 
-// rows per segment of the CN recurrences: 9 keeps a 129-plane column at 8
-// modes per CTA within four warps (15 segments), so that at the 128
-// registers a thread takes four CTAs share an SM (five warps fit three)
-constexpr int SEG_K = 9;
-constexpr int COL_MAX_THR = 256; // threads per CTA: MT x segments, rounded up to warps
+// Rows per segment: with 5 a thread's rows of all its inputs all but fit 128
+// registers (Re_tau = 180: 41 us per launch; 43 with 4, 55 with 3; 54 with 7 and 65
+// with 9, which spill); with 3 a short column takes less code, and time, to
+// start up (64x33x16: 10.6 us, 14.6 with 5).
+constexpr int SEG_K = 5, SEG_KS = 3, SEG_SHORT = 48;  // 3 up to 48 rows
+constexpr int COL_MAX_THR = 512; // threads per CTA: MT x segments, rounded up to warps
 
 struct ColConst {
   int NY, nf, nth, nkxp, JS, JE;
@@ -67,17 +74,15 @@ struct ColConst {
   double ri[DG_MAX_TH], pr[DG_MAX_TH], drhodx[DG_MAX_TH], drhodz[DG_MAX_TH];
 };
 
-// Everything the column stage of one case needs, in device memory (tensor
-// maps first: 64-byte aligned).  Maps are 2-D over [plane][2 ss doubles].
+// Everything the column stage of one case needs, in device memory.
 struct ColCase {
-  CUtensorMap map_cu[3 + DG_MAX_TH], map_nl[3 + DG_MAX_TH];
   ColConst C;
   const double *dscal, *tab, *kxv, *kzv, *rowc;
   const double2 *cp;
-  const double2 *cu[3 + DG_MAX_TH];
+  const double2 *cu[3 + DG_MAX_TH], *nl[3 + DG_MAX_TH];
   double2 *cf[3 + DG_MAX_TH], *out[3 + DG_MAX_TH];  // out: the rhs arrays
   int *err;
-  int by, nbox, nseg;
+  int nseg;
 };
 
 template <typename T>
@@ -97,20 +102,17 @@ __device__ __forceinline__ double2 z2() { return make_double2(0.0, 0.0); }
 //   4 1/DY(j)             5 DYF(j)                 (U2)
 //   6 1/DYF(j)            7 REM_DIV upper diagonal
 
-// The field's coefficients that do not change along the column.
-// Everything the right-hand side of one field needs besides the tiles, read
-// from the case table once per CTA into registers (the loop that uses them
-// stores to global memory, after which the compiler would have to reload
-// anything it reads from the table).
+// The field's coefficients that do not change along the column, read from the
+// case table once per CTA.  What other fields add to the explicit terms at row j
+// is linear in them: sum_q w[q] X_q(j) over src[q] (U1, U3: rotation and RI
+// GRAV_x/z TH; U2: RI GRAV_y TH, then interpolated to GY; a scalar: -DRHODX U1 - DRHODZ U3).
 struct FieldCoef {
-  double T3, T4, T5, aaU, NU, nup, ipr, ddx, ddz, sgn, time;
-  double i_ro, px0, amp_omega0, omega0;
-  double w[DG_MAX_TH];              // coupling weight of each scalar (0: none)
-  const double2 *th[DG_MAX_TH];     // the scalars' CU
-  const double2 *uo;                // the other horizontal velocity (rotation)
-  const double2 *u1, *u3;           // U1, U3 (DRHODX/Z in a scalar's equation)
-  long ss;
-  int lo, hi, nth, f_type;
+  double T3, T4, T5, aa, nu;
+  double force;                     // T4 times the mean pressure gradient (U1)
+  double w[1 + DG_MAX_TH];
+  const double2 *src[1 + DG_MAX_TH];
+  int nsrc;                         // 0: nothing couples
+  int lo, hi;
 };
 
 __device__ __forceinline__ FieldCoef field_coef(const ColCase &cc, int rk_step, int f) {
@@ -119,401 +121,374 @@ __device__ __forceinline__ FieldCoef field_coef(const ColCase &cc, int rk_step, 
   const double h = cc.dscal[1 + rk_step];
   const double zeta = (rk_step == 2) ? -17.0 / 8.0 : (rk_step == 3) ? -5.0 / 4.0 : 0.0;
   const double bbar = (rk_step == 2) ? 25.0 / 8.0 : (rk_step == 3) ? 9.0 / 4.0 : 1.0;
-  const double T1 = C.nu * h / 2.0;
   k.T3 = zeta * h;
   k.T4 = h;
   k.T5 = bbar * h;
-  k.aaU = T1 * C.nuv;
-  k.NU = C.nu;
-  k.time = cc.dscal[0];
   const int n = f - 3;
-  k.nup = (f >= 3) ? C.nu / pick(C.pr, n) : C.nu;
-  k.ipr = (f >= 3) ? 1.0 / pick(C.pr, n) : 1.0;
-  k.ddx = (f >= 3) ? pick(C.drhodx, n) : 0.0;
-  k.ddz = (f >= 3) ? pick(C.drhodz, n) : 0.0;
-  k.sgn = (f == 0) ? 1.0 : -1.0;
-  k.i_ro = C.i_ro;
-  k.px0 = C.px0;
-  k.amp_omega0 = C.amp_omega0;
-  k.omega0 = C.omega0;
-  k.f_type = C.f_type;
-  k.nth = C.nth;
-  k.ss = C.ss;
-  // U1, U3: RI GRAV_x/z TH; U2: RI GRAV_y times the GY interpolation
-  const double gr = (f == 0) ? C.grav_x : (f == 2) ? C.grav_z : C.grav_y;
+  const double ipr = (f >= 3) ? 1.0 / pick(C.pr, n) : 1.0;
+  k.nu = (f >= 3) ? C.nu / pick(C.pr, n) : C.nu;
+  k.aa = ipr * ((C.nu * h / 2.0) * C.nuv);
+  k.force = 0.0;
+  if (f == 0 && C.f_type == 1) k.force = k.T4 * C.px0;
+  else if (f == 0 && C.f_type == 2)
+    k.force = k.T4 * (C.px0 + C.amp_omega0 * cos(C.omega0 * cc.dscal[0]));
+  k.nsrc = 0;
 #pragma unroll
-  for (int q = 0; q < DG_MAX_TH; q++) {
-    k.w[q] = (q < C.nth && f < 3) ? C.ri[q] * gr : 0.0;
-    k.th[q] = cc.cu[3 + (q < C.nth ? q : 0)];
+  for (int q = 0; q <= DG_MAX_TH; q++) {
+    k.w[q] = 0.0;
+    k.src[q] = cc.cu[0];
   }
-  k.uo = cc.cu[(f == 0) ? 2 : 0];
-  k.u1 = cc.cu[0];
-  k.u3 = cc.cu[2];
+  if (f >= 3) {
+    k.w[0] = -pick(C.drhodx, n);
+    k.w[1] = -pick(C.drhodz, n);
+    k.src[1] = cc.cu[2];
+    if (k.w[0] != 0.0 || k.w[1] != 0.0) k.nsrc = 2;
+  } else {
+    const double gr = (f == 0) ? C.grav_x : (f == 2) ? C.grav_z : C.grav_y;
+    k.w[0] = (f == 0) ? C.i_ro : (f == 2) ? -C.i_ro : 0.0;
+    k.src[0] = cc.cu[(f == 0) ? 2 : 0];
+    if (k.w[0] != 0.0) k.nsrc = 1;
+#pragma unroll
+    for (int q = 0; q < DG_MAX_TH; q++) {
+      if (q >= C.nth) break;
+      k.w[1 + q] = C.ri[q] * gr;
+      k.src[1 + q] = cc.cu[3 + q];
+      if (k.w[1 + q] != 0.0) k.nsrc = 2 + q;
+    }
+  }
   if (f == 0 || f == 2) { k.lo = C.JS; k.hi = C.JE; }
   else if (f == 1) { k.lo = 2; k.hi = C.NY; }
   else { k.lo = pick(C.JSt, n); k.hi = pick(C.JEt, n); }
   return k;
 }
 
-// The explicit terms fv (the new CF) and the CN right-hand side r of field f
-// at row j, mode offset o: u, um, up = CU at j, j-1, j+1; nlv = NL;
-// old = CF_old; p0, pm = CP at j, j-1.  RC: the field's grid-factor rows in
-// shared memory, row stride ld: rows 0, 1 (U1, U3, TH) or 2, 3, 4, 5 (U2).
-template <int FK>
-__device__ __forceinline__ void rhs_row(const FieldCoef &k, int f, int j, long o, bool mean,
-                                        double KX, double KZ, double kk, const double *RC, int ld,
-                                        double2 u, double2 um, double2 up, double2 nlv,
-                                        double2 old, double2 p0, double2 pm, double2 &fv,
-                                        double2 &r) {
-  if constexpr (FK == 0) {
-    fv = make_double2(-k.NU * kk * u.x, -k.NU * kk * u.y);
-    if (k.i_ro != 0.0) {
-      const double2 uo = k.uo[o];
-      fv.x += k.sgn * k.i_ro * uo.x;
-      fv.y += k.sgn * k.i_ro * uo.y;
-    }
-#pragma unroll
-    for (int q = 0; q < DG_MAX_TH; q++) {
-      const double w = k.w[q];
-      if (q >= k.nth || w == 0.0) continue;
-      const double2 t = k.th[q][o];
-      fv.x += w * t.x;
-      fv.y += w * t.y;
-    }
-    fv.x += nlv.x;
-    fv.y += nlv.y;
-    r = u;
-    r.x += k.T3 * old.x;
-    r.y += k.T3 * old.y;
-    const double K = (f == 0) ? KX : KZ;
-    r.x -= k.T4 * (-K * p0.y);
-    r.y -= k.T4 * (K * p0.x);
-    if (f == 0 && mean) {
-      if (k.f_type == 1) r.x -= k.T4 * k.px0;
-      else if (k.f_type == 2) r.x -= k.T4 * (k.px0 + k.amp_omega0 * cos(k.omega0 * k.time));
-    }
-    r.x += k.T5 * fv.x;
-    r.y += k.T5 * fv.y;
-    const double cup = k.aaU * RC[0 * ld + j], cdn = k.aaU * RC[1 * ld + j];
-    r.x += cup * (up.x - u.x) - cdn * (u.x - um.x);
-    r.y += cup * (up.y - u.y) - cdn * (u.y - um.y);
-  } else if constexpr (FK == 1) {
-    fv = make_double2(-k.NU * kk * u.x, -k.NU * kk * u.y);
-    if (!mean) {
-      const double dyfj = RC[3 * ld + j], dyfm = RC[3 * ld + j - 1];
-      const double bw2 = 0.5 * RC[2 * ld + j];
-#pragma unroll
-      for (int q = 0; q < DG_MAX_TH; q++) {
-        if (q >= k.nth || k.w[q] == 0.0) continue;
-        const double w = k.w[q] * bw2;
-        const double2 t = k.th[q][o], tm = k.th[q][o - k.ss];
-        fv.x += w * (t.x * dyfm + tm.x * dyfj);
-        fv.y += w * (t.y * dyfm + tm.y * dyfj);
-      }
-    }
-    fv.x += nlv.x;
-    fv.y += nlv.y;
-    r = u;
-    r.x += k.T3 * old.x;
-    r.y += k.T3 * old.y;
-    const double idy = RC[2 * ld + j];
-    r.x -= k.T4 * ((p0.x - pm.x) * idy);
-    r.y -= k.T4 * ((p0.y - pm.y) * idy);
-    r.x += k.T5 * fv.x;
-    r.y += k.T5 * fv.y;
-    const double cup2 = k.aaU * RC[0 * ld + j], cdn2 = k.aaU * RC[1 * ld + j];
-    r.x += cup2 * (up.x - u.x) - cdn2 * (u.x - um.x);
-    r.y += cup2 * (up.y - u.y) - cdn2 * (u.y - um.y);
-  } else {
-    fv = make_double2(-k.nup * kk * u.x, -k.nup * kk * u.y);
-    if (k.ddx != 0.0 || k.ddz != 0.0) {
-      const double2 u1 = k.u1[o], u3 = k.u3[o];
-      fv.x = fv.x - u1.x * k.ddx - u3.x * k.ddz;
-      fv.y = fv.y - u1.y * k.ddx - u3.y * k.ddz;
-    }
-    fv.x += nlv.x;
-    fv.y += nlv.y;
-    r = u;
-    r.x += k.T3 * old.x;
-    r.y += k.T3 * old.y;
-    r.x += k.T5 * fv.x;
-    r.y += k.T5 * fv.y;
-    const double cup = k.aaU * RC[0 * ld + j], cdn = k.aaU * RC[1 * ld + j];
-    r.x += k.ipr * (cup * (up.x - u.x) - cdn * (u.x - um.x));
-    r.y += k.ipr * (cup * (up.y - u.y) - cdn * (u.y - um.y));
-  }
-}
-
 // Launch-wide sizes: the largest item of the work list sets the layout.
 struct ColLaunch {
-  int tile;   // double2 per tile (nbox * by * MT of the largest case)
   int lp;     // table row length (the largest case's NY + 2, rounded up to even)
-  int nseg;   // segments per column (the largest case)
   int nwork;  // work items (CTAs)
 };
 
-// Shared memory of one CTA (128-byte aligned): the tiles CU and NL (then R,
-// g, e and x of the recurrences) [tile] double2; the CN table
-// rows TB [5][lp] (a, 1/b, f = -c/b, kind, BC value); the field's grid
-// factors RC [4][lp]; per (segment, mode) values SV [nseg][MT] double2
-// (then carries); per segment products SP [nseg]; the modes' wavenumbers
-// and k^2 (to the power BETA) KW [3][MT]; the mbarrier.
-size_t col_smem_l(const ColLaunch &P, int mt) {
-  return sizeof(double2) * (2 * (size_t)P.tile + (size_t)P.nseg * mt) +
-         sizeof(double) * (9 * (size_t)P.lp + (size_t)P.nseg + 3 * (size_t)mt) + 8 + 128;
+// Shared memory of one CTA: the CN table rows TB [5][lp] (a, 1/b, f = -c/b,
+// kind, BC value); the field's grid factors RC [4][lp]; the totals of the quads (pairs) of
+// segments for the two directions, end values TG [2][pairs][MT] double2 and products
+// TP [2][pairs]; the mbarrier.
+size_t col_smem_l(const ColLaunch &P, int mt, int thr) {
+  const size_t pairs = thr / (2 * mt);
+  return sizeof(double) * (9 * (size_t)P.lp + 2 * pairs * (2 * mt + 1)) + 16;
 }
 
-// The right-hand side of field f (kind FK: 0 U1/U3, 1 U2, 2 scalar) for the
-// CTA's rows lo..hi: a flat loop over (row, mode) elements in batches of
-// four per thread; CU and NL from the staged tiles, CF_old and CP read
-// directly (each element once, coalesced).  CF_old is the array the loop
-// writes CF into, so a batch's loads are all issued before its stores; CP
-// is read-only here and goes through the read-only data path.  R replaces
-// NL.  Everything else the loop reads is in registers or shared memory.
-template <int MT, int FK>
-__device__ __forceinline__ void rhs_tile(const FieldCoef &k, int rk_step, long m0, int f, int mt,
-                                         double2 *cff, const double2 *cpp, const double2 *CUt,
-                                         double2 *NLt, const double *RC, int LP,
-                                         const double *KW) {
-  const bool old_cf = rk_step > 1;
-  const int nthr = blockDim.x;
-  const int i0 = k.lo * MT + (int)threadIdx.x, iend = (k.hi + 1) * MT;
-  constexpr int B = 4;
-  for (int base = i0; base < iend; base += B * nthr) {
-    double2 old[B], p0[B], pm[B];
-#pragma unroll
-    for (int u = 0; u < B; u++) {
-      const int i = base + u * nthr;
-      const int j = i / MT, m = i - j * MT;
-      const bool ok = i < iend && m < mt;
-      const long o = (long)j * k.ss + m0 + m;
-      old[u] = (ok && old_cf) ? cff[o] : z2();
-      p0[u] = (ok && FK < 2) ? __ldg(cpp + o) : z2();
-      pm[u] = (ok && FK == 1) ? __ldg(cpp + o - k.ss) : z2();
+// What enters segment s of mode m from the segments before it (DIR = +1: rows
+// above in index order; -1: from the last one back): the states (end value e, product p) of
+// the segments compose as e2 + p2 X, (e, p) per segment, identity (0, 1) where a thread has no
+// rows.  Segments go in pairs and quads (a fixed order, so that the result does not depend on
+// the tile width): by shuffles inside a warp, which holds 32 / MT segments, the
+// totals of the quads (of the pairs for MT = 16) in shared memory, then quad by quad.
+template <int MT, int DIR>
+__device__ __forceinline__ double2 carry(int s, int m, int nseg, double2 e, double p, double2 *TG,
+                                         double *TP) {
+  static_assert(MT <= 16, "the two segments of a pair share a warp");
+  constexpr unsigned ALL = 0xffffffffu;
+  const bool late = DIR > 0 ? (s & 1) : !(s & 1);      // second of its pair
+  const bool late2 = DIR > 0 ? (s & 2) : !(s & 2);     // in the second pair of its quad
+  const int lane = threadIdx.x & 31;
+  // the pair
+  const int src1 = lane ^ MT;
+  const double2 o = make_double2(__shfl_sync(ALL, e.x, src1), __shfl_sync(ALL, e.y, src1));
+  const double op = __shfl_sync(ALL, p, src1);
+  double2 c = late ? o : z2();
+  double pe = late ? op : 1.0;
+  // the pair's total (right in its second segment)
+  e = make_double2(e.x + p * o.x, e.y + p * o.y);
+  p = p * op;
+  if constexpr (MT <= 8) {
+    // the first pair's total, from its second segment
+    const int sw = lane / MT, q0 = sw & ~3;
+    const int src2 = (q0 + (DIR > 0 ? 1 : 2)) * MT + m;
+    const double2 t = make_double2(__shfl_sync(ALL, e.x, src2), __shfl_sync(ALL, e.y, src2));
+    const double tp = __shfl_sync(ALL, p, src2);
+    if (late2) {
+      c = make_double2(c.x + pe * t.x, c.y + pe * t.y);
+      pe = pe * tp;
     }
+    if (late && late2) {
+      TG[(s >> 2) * MT + m] = make_double2(e.x + p * t.x, e.y + p * t.y);
+      if (m == 0) TP[s >> 2] = p * tp;
+    }
+  } else if (late) {
+    TG[(s >> 1) * MT + m] = e;
+    if (m == 0) TP[s >> 1] = p;
+  }
+  __syncthreads();
+  const int quad = s >> 2, npair = blockDim.x / (2 * MT);
+  if constexpr (MT > 8) {
+    if (late2) {
+      // the pair before this one (it may lie beyond the CTA's last thread)
+      const int w = 2 * quad + (DIR > 0 ? 0 : 1);
+      const double2 t = w < npair ? TG[w * MT + m] : z2();
+      c = make_double2(c.x + pe * t.x, c.y + pe * t.y);
+      pe = pe * (w < npair ? TP[w] : 1.0);
+    }
+  }
+  // the quads before this one, four at a time (their loads ahead of the chain)
+  const int nq = DIR > 0 ? quad : ((nseg - 1) >> 2) - quad;
+  double2 X = z2();
+  for (int w0 = 0; w0 < nq; w0 += 4) {
+    double2 t[4];
+    double tp[4];
 #pragma unroll
-    for (int u = 0; u < B; u++) {
-      const int i = base + u * nthr;
-      const int j = i / MT, m = i - j * MT;
-      if (i < iend && m < mt) {
-        const long mg = m0 + m;
-        const long o = (long)j * k.ss + mg;
-        double2 fv, rr;
-        rhs_row<FK>(k, f, j, o, mg == 0, KW[m], KW[MT + m], KW[2 * MT + m], RC, LP, CUt[i],
-                    CUt[i - MT], CUt[i + MT], NLt[i], old[u], p0[u], pm[u], fv, rr);
-        cff[o] = fv;
-        NLt[i] = rr;
+    for (int i = 0; i < 4; i++) {
+      const int w = DIR > 0 ? w0 + i : ((nseg - 1) >> 2) - w0 - i;
+      t[i] = z2();
+      tp[i] = 1.0;
+      if (w0 + i < nq) {
+        if constexpr (MT <= 8) {
+          t[i] = TG[w * MT + m];
+          tp[i] = TP[w];
+        } else {
+          const int a = 2 * w + (DIR > 0 ? 0 : 1), b = 2 * w + (DIR > 0 ? 1 : 0);  // first, second
+          const double2 ta = a < npair ? TG[a * MT + m] : z2(), tb = b < npair ? TG[b * MT + m] : z2();
+          const double pa = a < npair ? TP[a] : 1.0, pb = b < npair ? TP[b] : 1.0;
+          t[i] = make_double2(tb.x + pb * ta.x, tb.y + pb * ta.y);
+          tp[i] = pb * pa;
+        }
       }
     }
+#pragma unroll
+    for (int i = 0; i < 4; i++) X = make_double2(t[i].x + tp[i] * X.x, t[i].y + tp[i] * X.y);
+  }
+  return make_double2(c.x + pe * X.x, c.y + pe * X.y);
+}
+
+// The column stage of field f (kind FK: 0 U1/U3, 1 U2, 2 scalar): explicit
+// terms, CF, R and the CN solve of the thread's rows j0 .. j0+nr-1 of one mode,
+// whose row 0 lies at offset mg of every field.
+template <int MT, int K, int FK, bool CPL, typename Table>
+__device__ __forceinline__ void col_rows(const FieldCoef &k, bool old_cf, int L, long ss, long mg,
+                                         int j0, int nr, int nseg, bool mean, double Kh, double kk,
+                                         int wlo,
+                                         const double2 *__restrict__ cu, const double2 *nl,
+                                         double2 *cff, const double2 *__restrict__ cpp,
+                                         double2 *dst, const double *TB, const double *RC, int LP,
+                                         double2 *TG, double *TP, Table table) {
+  const int s = threadIdx.x / MT, m = threadIdx.x % MT;
+  const int slots = blockDim.x / (2 * MT);
+  const long o0 = (long)j0 * ss + mg;
+  auto in = [&](int q) { return q < nr && j0 + q >= k.lo && j0 + q <= k.hi; };
+  // ---- 1. R.  Every input row is on its way before the first is used, and
+  // before the wait for the table rows.
+  double2 r[K], p[K + 1], u[K + 2], v[K];  // CF_old, CP rows j0-1 .., CU rows j0-1 .., NL
+#pragma unroll
+  for (int q = 0; q < K; q++) r[q] = (old_cf && in(q)) ? cff[o0 + q * ss] : z2();
+  if (FK < 2) {
+#pragma unroll
+    for (int q = 0; q < K; q++) p[q + 1] = in(q) ? __ldg(cpp + o0 + q * ss) : z2();
+  }
+  if (FK == 1) p[0] = (nr > 0 && j0 > 0) ? __ldg(cpp + o0 - ss) : z2();
+#pragma unroll
+  for (int q = 0; q < K + 2; q++) {
+    const int j = j0 + q - 1;
+    u[q] = (nr > 0 && j >= 0 && j < L) ? __ldg(cu + o0 + (q - 1) * ss) : z2();
+  }
+#pragma unroll
+  for (int q = 0; q < K; q++) v[q] = in(q) ? nl[o0 + q * ss] : z2();
+  if (!table()) return;
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    r[q].x *= k.T3;
+    r[q].y *= k.T3;
+    if (FK == 0) {
+      // - h (i K P), Kh = h K
+      r[q].x += Kh * p[q + 1].y;
+      r[q].y -= Kh * p[q + 1].x;
+    } else if (FK == 1 && in(q)) {
+      const double c = k.T4 * RC[2 * LP + j0 + q];
+      r[q].x -= c * (p[q + 1].x - p[q].x);
+      r[q].y -= c * (p[q + 1].y - p[q].y);
+    }
+  }
+  {
+    // what other fields add (w X summed over the fields)
+    auto others = [&](int q) -> double2 {
+      double2 S = z2();
+#pragma unroll
+      for (int e = 0; e <= DG_MAX_TH; e++) {
+        if (e >= k.nsrc) break;
+        if (k.w[e] == 0.0) continue;
+        const double2 x = __ldg(k.src[e] + o0 + q * ss);
+        S.x += k.w[e] * x.x;
+        S.y += k.w[e] * x.y;
+      }
+      return S;
+    };
+    double2 Sm = z2();
+    if (CPL && FK == 1 && nr > 0 && j0 > 0) Sm = others(-1);
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+      double2 S = z2();
+      if (CPL && q < nr) S = others(q);
+      if (in(q)) {
+        const int j = j0 + q;
+        const double2 uc = u[q + 1];
+        double2 fv = make_double2(-k.nu * kk * uc.x, -k.nu * kk * uc.y);
+        if (FK == 1) {
+          if (CPL && !mean) {
+            const double dyfj = RC[3 * LP + j], dyfm = RC[3 * LP + j - 1];
+            const double bw2 = 0.5 * RC[2 * LP + j];
+            fv.x += bw2 * (S.x * dyfm + Sm.x * dyfj);
+            fv.y += bw2 * (S.y * dyfm + Sm.y * dyfj);
+          }
+        } else if (CPL) {
+          fv.x += S.x;
+          fv.y += S.y;
+        }
+        fv.x += v[q].x;
+        fv.y += v[q].y;
+        cff[o0 + q * ss] = fv;
+        r[q].x += uc.x;
+        r[q].y += uc.y;
+        if (FK == 0 && mean) r[q].x -= k.force;
+        r[q].x += k.T5 * fv.x;
+        r[q].y += k.T5 * fv.y;
+        const double cup = k.aa * RC[j], cdn = k.aa * RC[LP + j];
+        r[q].x += cup * (u[q + 2].x - uc.x) - cdn * (uc.x - u[q].x);
+        r[q].y += cup * (u[q + 2].y - uc.y) - cdn * (uc.y - u[q].y);
+      }
+      Sm = S;
+    }
+  }
+  // ---- 2. the forward recurrence from zero; the right-hand side is R on CN
+  // rows, the BC value (the (0,0) mode's real part) or zero elsewhere
+  double2 g = z2();
+  double pa = 1.0;
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    if (q < nr) {
+      const int j = j0 + q;
+      const double kind = TB[3 * LP + j], a = TB[j];
+      if (kind != (double)ROW_RHS)
+        r[q] = make_double2((kind == (double)ROW_BC && mean) ? TB[4 * LP + j] : 0.0, 0.0);
+      g.x = r[q].x + a * g.x;
+      g.y = r[q].y + a * g.y;
+      pa = a * pa;
+      r[q] = g;
+    }
+  }
+  // ---- 3. the segment ends carried down the column
+  double2 c = carry<MT, +1>(s, m, nseg, make_double2(g.x, g.y), pa, TG, TP);
+  // ---- 4. g = local + product x carry, e = g / b; then the backward
+  // recurrence x(j) = e(j) + f(j) x(j+1) over the segment (rows >= wlo)
+  double pi = 1.0;
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    if (q < nr) {
+      pi = TB[j0 + q] * pi;
+      const double rb = TB[LP + j0 + q];
+      r[q] = make_double2((r[q].x + pi * c.x) * rb, (r[q].y + pi * c.y) * rb);
+    }
+  }
+  const int qb = wlo > j0 ? wlo - j0 : 0;  // first row of the segment to solve
+  double2 xl = z2();
+  double ps = 1.0;
+#pragma unroll
+  for (int q = K - 1; q >= 0; q--) {
+    if (q < nr && q >= qb) {
+      const double fc = TB[2 * LP + j0 + q];
+      xl = make_double2(r[q].x + fc * xl.x, r[q].y + fc * xl.y);
+      ps = fc * ps;
+      r[q] = xl;
+    }
+  }
+  // ---- 5. the segment starts carried up the column
+  c = carry<MT, -1>(s, m, nseg, xl, ps, TG + slots * MT, TP + slots);
+  // ---- 6. x = local + product x carry: the post-CN field, rows >= wlo
+  double p2 = 1.0;
+#pragma unroll
+  for (int q = K - 1; q >= 0; q--) {
+    if (q < nr && q >= qb) {
+      p2 = TB[2 * LP + j0 + q] * p2;
+      dst[o0 + q * ss] = make_double2(r[q].x + p2 * c.x, r[q].y + p2 * c.y);
+    }
   }
 }
 
-// Carry the per-segment values e(t) through the segments in order
-// t = t0, t0 + dt, ..., n steps: X(t) = e(t) + p(t) X(previous), storing the
-// carry into each segment (its value before the segment) in place of e(t).
-template <int MT>
-__device__ __forceinline__ void carry_chain(double2 *SV, const double *SP, int t0, int dt, int n,
-                                            int m) {
-  double2 X = z2();
-  for (int b = 0; b < n; b++) {
-    const int t = t0 + dt * b;
-    const double2 e = SV[t * MT + m];
-    const double p = SP[t];
-    SV[t * MT + m] = X;
-    X = make_double2(e.x + p * X.x, e.y + p * X.y);
-  }
-}
-
-// The column stage of field f for modes m0 .. m0+MT-1 of one case.  Every
-// value the CTA needs from the case table is read before its first global
-// store (after which the compiler would have to reload it).
-template <int MT>
+// The column stage of field f for modes m0 .. m0+MT-1 of one case.
+template <int MT, int K>
 __device__ __forceinline__ void col_body(const ColCase &cc, int rk_step, long m0, int f,
                                          const ColLaunch &P, long spin, unsigned extra_tx,
-                                         unsigned char *sbase) {
+                                         double *sbase) {
   const int NY = cc.C.NY, L = NY + 2, LP = (L + 1) & ~1;  // the case's own row length
-  const int nseg = cc.nseg;
   const long ss = cc.C.ss;
   const int mt = (int)((ss - m0) < MT ? (ss - m0) : MT);
   const int wlo = (f >= 3) ? pick(cc.C.JSt, f - 3) - 1 : 1;  // first row solved
-  double2 *const dst = cc.out[f];
-  double2 *const cff = cc.cf[f];
-  int *const err = cc.err;
-  const FieldCoef k = field_coef(cc, rk_step, f);
-  double2 *CUt = reinterpret_cast<double2 *>(sbase);
-  double2 *NLt = CUt + P.tile;
-  double *TB = reinterpret_cast<double *>(NLt + P.tile);
-  const double2 *const cpp = cc.cp;
+  double *TB = sbase;
   double *RC = TB + 5 * P.lp;  // the slots are sized for the largest case
-  double2 *SV = reinterpret_cast<double2 *>(RC + 4 * P.lp);
-  double *SP = reinterpret_cast<double *>(SV + P.nseg * MT);
-  double *KW = SP + P.nseg;
-  unsigned long long *bar = reinterpret_cast<unsigned long long *>(KW + 3 * MT);
-  const int tid = threadIdx.x;
-  if (tid < MT) {
-    const long mg = (m0 + tid < ss) ? m0 + tid : 0;
-    const double KX = cc.kxv[mg % cc.C.nkxp], KZ = cc.kzv[mg / cc.C.nkxp];
-    const double k2 = KX * KX + KZ * KZ;
-    KW[tid] = KX;
-    KW[MT + tid] = KZ;
-    KW[2 * MT + tid] = (cc.C.beta == 1.0) ? k2 : pow(k2, cc.C.beta);
-  }
-
-  // ---- 0. the field's tiles by bulk tensor copies, the table and grid-
-  // factor rows by bulk copies, all in flight at once on one mbarrier
+  double2 *TG = reinterpret_cast<double2 *>(RC + 4 * P.lp);
+  const int tid = threadIdx.x, npair = blockDim.x / (2 * MT);
+  double *TP = reinterpret_cast<double *>(TG + 2 * npair * MT);
+  unsigned long long *bar = reinterpret_cast<unsigned long long *>(TP + 2 * npair);
+  // the table and grid-factor rows by bulk copies on one mbarrier
   if (tid == 0) dg_mbar_init(bar, 1);
   __syncthreads();
   dg_pdl_wait();  // NL comes from the z-forward kernel
   if (tid == 0) {
-    const int ctile = cc.nbox * cc.by * MT;
-    const unsigned ntiles = 2u;
     const int nrc = (f == 1) ? 4 : 2;  // grid-factor rows 2..5 (U2) or 0..1
     // extra_tx is 0 except in the wait test, where the barrier then never completes
-    dg_mbar_expect_tx(bar, (unsigned)(sizeof(double2) * ctile) * ntiles +
-                               (unsigned)(sizeof(double) * (5 + nrc) * LP) + extra_tx);
-    // columns beyond ss and planes beyond L arrive as zeros
-    for (int q = 0; q < cc.nbox; q++) {
-      const long d = (long)q * cc.by * MT;
-      const int x = (int)(2 * m0), y = q * cc.by;
-      dg_tma_load_2d(CUt + d, &cc.map_cu[f], x, y, bar);
-      dg_tma_load_2d(NLt + d, &cc.map_nl[f], x, y, bar);
-    }
+    dg_mbar_expect_tx(bar, (unsigned)(sizeof(double) * (5 + nrc) * LP) + extra_tx);
     dg_bulk_load(TB, cc.tab + ((long)(rk_step - 1) * (3 + DG_MAX_TH) + f) * 5 * LP,
                  (unsigned)(sizeof(double) * 5 * LP), bar);
     dg_bulk_load(RC, cc.rowc + (long)(f == 1 ? 2 : 0) * LP,
                  (unsigned)(sizeof(double) * nrc * LP), bar);
   }
-  const bool landed = dg_mbar_wait(bar, 0, spin);
-  if (__syncthreads_or(!landed)) {
-    if (tid == 0) {
-      atomicExch(err + 1, 1);
-      dg_mbar_wait(bar, 0, spin);  // the copies in flight get one more bounded wait
-    }
-    return;
-  }
-
-  // ---- 1. explicit terms, CF and the right-hand side of rows lo..hi
-  if (f == 1) rhs_tile<MT, 1>(k, rk_step, m0, f, mt, cff, cpp, CUt, NLt, RC, LP, KW);
-  else if (f < 3) rhs_tile<MT, 0>(k, rk_step, m0, f, mt, cff, cpp, CUt, NLt, RC, LP, KW);
-  else rhs_tile<MT, 2>(k, rk_step, m0, f, mt, cff, cpp, CUt, NLt, RC, LP, KW);
-  __syncthreads();
-
-  // ---- 2. forward recurrence g(j) = r(j) + a(j) g(j-1) over each segment
-  // from zero (one thread per mode and segment); r is R on CN rows, the BC
-  // value (the (0,0) mode's real part) or zero elsewhere; g replaces R.
-  // Each phase loads its rows first, then runs its chain.
   const int m = tid % MT, s = tid / MT;
-  const int j0 = s * SEG_K;
-  const int nr = (s < nseg) ? min(SEG_K, L - j0) : 0;  // rows of this thread's segment
-  const long mg = m0 + m;
-  const bool live = m < mt;
-  const bool mean = (mg == 0);
-  double a[SEG_K];
-  {
-    double2 r[SEG_K];
-#pragma unroll
-    for (int q = 0; q < SEG_K; q++) {
-      const int j = (q < nr) ? j0 + q : 0;
-      const double kind = TB[3 * LP + j];
-      const double2 rv = NLt[j * MT + m];
-      const double bc = TB[4 * LP + j];
-      r[q] = (kind == (double)ROW_RHS)
-                 ? rv
-                 : make_double2((kind == (double)ROW_BC && mean) ? bc : 0.0, 0.0);
-      a[q] = TB[j];
-    }
-    double2 g = z2();
-    double pa = 1.0;
-#pragma unroll
-    for (int q = 0; q < SEG_K; q++) {
-      if (q < nr) {
-        g.x = r[q].x + a[q] * g.x;
-        g.y = r[q].y + a[q] * g.y;
-        pa = a[q] * pa;
-        NLt[(j0 + q) * MT + m] = g;
+  const int nseg = cc.nseg;
+  const bool mine = m < mt && s < nseg;
+  const long mg = m < mt ? m0 + m : m0;
+  const int j0 = s * K, nr = mine ? min(K, L - j0) : 0;
+  const double2 *cu = cc.cu[f], *nl = cc.nl[f], *cpp = cc.cp;
+  double2 *cff = cc.cf[f], *dst = cc.out[f];
+  int *err = cc.err;
+  const FieldCoef k = field_coef(cc, rk_step, f);
+  const double KX = cc.kxv[mg % cc.C.nkxp], KZ = cc.kzv[mg / cc.C.nkxp];
+  const double k2 = KX * KX + KZ * KZ;
+  const double kk = (cc.C.beta == 1.0) ? k2 : pow(k2, cc.C.beta);
+  const double Kh = k.T4 * ((f == 2) ? KZ : KX);
+  // the table rows have landed (false: they did not within the wait limit)
+  auto table = [&]() -> bool {
+    const bool landed = dg_mbar_wait(bar, 0, spin);
+    if (__syncthreads_or(!landed)) {
+      if (tid == 0) {
+        atomicExch(err + 1, 1);
+        dg_mbar_wait(bar, 0, spin);  // the copies in flight get one more bounded wait
       }
+      return false;
     }
-    if (nr > 0) {
-      SV[s * MT + m] = g;
-      if (m == 0) SP[s] = pa;
-    }
+    return true;
+  };
+  const bool old_cf = rk_step > 1;
+#define COL_ROWS(FK, CPL)                                                                     \
+  col_rows<MT, K, FK, CPL>(k, old_cf, L, ss, mg, j0, nr, nseg, mg == 0, Kh, kk, wlo, cu, nl, cff, \
+                        cpp, dst, TB, RC, LP, TG, TP, table)
+  if (k.nsrc == 0) {
+    if (f == 1) COL_ROWS(1, false);
+    else if (f < 3) COL_ROWS(0, false);
+    else COL_ROWS(2, false);
+  } else {
+    if (f == 1) COL_ROWS(1, true);
+    else if (f < 3) COL_ROWS(0, true);
+    else COL_ROWS(2, true);
   }
-  __syncthreads();
-  // ---- 3. the segment ends carried down the column, one lane per mode
-  if (tid < MT) carry_chain<MT>(SV, SP, 0, 1, nseg, tid);
-  __syncthreads();
-  // ---- 4. g = local + product x carry, e = g / b; then the backward
-  // recurrence x(j) = e(j) + f(j) x(j+1) over the segment (rows >= wlo)
-  const int qb = wlo > j0 ? wlo - j0 : 0;  // first row of the segment to solve
-  const bool solves = nr > 0 && qb < nr;
-  double fc[SEG_K];
-  {
-    const double2 c = (nr > 0) ? SV[s * MT + m] : z2();
-    double2 e[SEG_K];
-    double rb[SEG_K];
-#pragma unroll
-    for (int q = 0; q < SEG_K; q++) {
-      const int j = (q < nr) ? j0 + q : 0;
-      e[q] = NLt[j * MT + m];
-      rb[q] = TB[LP + j];
-      fc[q] = TB[2 * LP + j];
-    }
-    double pi = 1.0;
-#pragma unroll
-    for (int q = 0; q < SEG_K; q++) {
-      pi = a[q] * pi;
-      e[q] = make_double2((e[q].x + pi * c.x) * rb[q], (e[q].y + pi * c.y) * rb[q]);
-    }
-    double2 xl = z2();
-    double ps = 1.0;
-#pragma unroll
-    for (int q = SEG_K - 1; q >= 0; q--) {
-      if (q < nr && q >= qb) {
-        xl = make_double2(e[q].x + fc[q] * xl.x, e[q].y + fc[q] * xl.y);
-        ps = fc[q] * ps;
-        NLt[(j0 + q) * MT + m] = xl;
-      }
-    }
-    // each thread overwrites only its own SV entry, read above by itself;
-    // SP was last read in step 3, before the barrier
-    if (solves) {
-      SV[s * MT + m] = xl;
-      if (m == 0) SP[s] = ps;
-    }
-  }
-  __syncthreads();
-  // ---- 5. the segment starts carried up the column, one lane per mode
-  const int sw = wlo / SEG_K;  // lowest segment with rows to solve
-  if (tid < MT) carry_chain<MT>(SV, SP, nseg - 1, -1, nseg - sw, tid);
-  __syncthreads();
-  // ---- 6. x = local + product x carry: the post-CN field, rows >= wlo
-  if (solves && live) {
-    const double2 c = SV[s * MT + m];
-    double2 xl[SEG_K];
-#pragma unroll
-    for (int q = 0; q < SEG_K; q++) xl[q] = NLt[((q < nr) ? j0 + q : 0) * MT + m];
-    double p2 = 1.0;
-#pragma unroll
-    for (int q = SEG_K - 1; q >= 0; q--) {
-      if (q < nr && q >= qb) {
-        p2 = fc[q] * p2;
-        dst[(long)(j0 + q) * ss + mg] = make_double2(xl[q].x + p2 * c.x, xl[q].y + p2 * c.y);
-      }
-    }
-  }
+#undef COL_ROWS
 }
 
 // The column kernel: CTA b takes work[b] = (case, mode tile, field) from
 // the case table (every case at substep rk_step with MT modes per CTA).
-template <int MT>
-__global__ void __launch_bounds__(COL_MAX_THR, 2) k_col_cn(const ColCase *__restrict__ cases,
-                                                       const int4 *__restrict__ work,
-                                                       ColLaunch P, int rk_step, long spin,
-                                                       unsigned extra_tx) {
-  extern __shared__ __align__(128) unsigned char cs_raw[];
-  unsigned char *sbase = cs_raw + ((128u - (dg_smem_addr(cs_raw) & 127u)) & 127u);
+template <int MT, int K>
+__global__ void __launch_bounds__(COL_MAX_THR)
+    k_col_cn(const ColCase *__restrict__ cases, const int4 *__restrict__ work, ColLaunch P,
+             int rk_step, long spin, unsigned extra_tx) {
+  extern __shared__ __align__(16) double cs_raw[];
   const int4 w = work[blockIdx.x];
-  col_body<MT>(cases[w.x], rk_step, (long)w.y * MT, w.z, P, spin, extra_tx, sbase);
+  col_body<MT, K>(cases[w.x], rk_step, (long)w.y * MT, w.z, P, spin, extra_tx, cs_raw);
 }
 
 ColConst make_col_const(const dg_handle *h) {
@@ -567,47 +542,29 @@ int dg_col_init(dg_handle *h) {
   return DG_OK;
 }
 
-static void col_geometry(const dg_handle *h, int *by, int *nbox, int *nseg) {
-  const int L = h->NY + 2;
-  // boxes of at most 256 planes; a multiple of 8 planes keeps every box's
-  // shared-memory destination 128-byte aligned for any modes per CTA
-  *nbox = dg_cdiv(L, 256);
-  *by = (dg_cdiv(L, *nbox) + 7) / 8 * 8;
-  *nseg = dg_cdiv(L, SEG_K);
+static int col_segk(const dg_handle *h) { return h->NY + 2 <= SEG_SHORT ? SEG_KS : SEG_K; }
+static int col_nseg(const dg_handle *h) { return dg_cdiv(h->NY + 2, col_segk(h)); }
+
+// threads of one CTA for handle h at mt modes: one per (mode, segment)
+static int col_threads(const dg_handle *h, int mt) {
+  return (mt * col_nseg(h) + 31) / 32 * 32;
 }
 
-// launch sizes of handle h alone at mt modes per CTA (nwork left 0)
-static ColLaunch col_sizes(const dg_handle *h, int mt) {
-  int by, nbox, nseg;
-  col_geometry(h, &by, &nbox, &nseg);
+// launch sizes of handle h alone (nwork left 0)
+static ColLaunch col_sizes(const dg_handle *h) {
   ColLaunch P;
-  P.tile = nbox * by * mt;
   P.lp = (h->NY + 2 + 1) / 2 * 2;
-  P.nseg = nseg;
   P.nwork = 0;
   return P;
 }
 
-// threads of one CTA for handle h at mt modes: one per (mode, segment), and
-// at least 128 for the flat right-hand-side loop
-static int col_threads(const dg_handle *h, int mt) {
-  return std::max(128, (mt * col_sizes(h, mt).nseg + 31) / 32 * 32);
+size_t dg_col_smem(const dg_handle *h, int mt) {
+  return col_smem_l(col_sizes(h), mt, col_threads(h, mt));
 }
 
-size_t dg_col_smem(const dg_handle *h, int mt) { return col_smem_l(col_sizes(h, mt), mt); }
-
-// The case description of handle h for `mt` modes per CTA (builds the
-// tensor maps of its CU and rhs arrays for that tile width).
-static int fill_case(dg_handle *h, int mt, ColCase *cc) {
-  const int L = h->NY + 2;
-  int by = 0, nbox = 0, nseg = 0;
-  col_geometry(h, &by, &nbox, &nseg);
+// the case description of handle h
+static void fill_case(dg_handle *h, ColCase *cc) {
   memset(cc, 0, sizeof(*cc));
-  for (int f = 0; f < h->nf; f++) {
-    DG_TRY(dg_tmap_planes(h->cu[f], h->ss, L, mt, by, &cc->map_cu[f]));
-    DG_TRY(dg_tmap_planes(h->rhs[f], h->ss, L, mt, by, &cc->map_nl[f]));
-  }
-  cc->cp = h->cp;
   cc->C = make_col_const(h);
   cc->dscal = h->dscal;
   cc->tab = h->cn_tab;
@@ -616,18 +573,17 @@ static int fill_case(dg_handle *h, int mt, ColCase *cc) {
   cc->rowc = h->rowc;
   for (int f = 0; f < h->nf; f++) {
     cc->cu[f] = h->cu[f];
+    cc->nl[f] = h->rhs[f];
     cc->cf[f] = h->cf[f];
     cc->out[f] = (f < 3 || dg_col_th_to_rhs(h, f - 3)) ? h->rhs[f] : h->cu[f];
   }
+  cc->cp = h->cp;
   cc->err = h->dflag;
-  cc->by = by;
-  cc->nbox = nbox;
-  cc->nseg = nseg;
-  return DG_OK;
+  cc->nseg = col_nseg(h);
 }
 
 // modes per CTA for handle h: the tuned value, halved until the CTA fits
-// (two stages in shared memory, one thread per mode and segment)
+// (one thread per mode and segment)
 static int col_mt(const dg_handle *h, int want) {
   int mt = want;
   while (mt > 2 && (dg_col_smem(h, mt) > 220 * 1024 || col_threads(h, mt) > COL_MAX_THR)) mt /= 2;
@@ -643,6 +599,8 @@ static int col_fits(const dg_handle *h, int mt) {
 }
 
 int dg_col_mt_eff(const dg_handle *h) { return col_mt(h, h->cn_mt); }
+
+int dg_col_class(const dg_handle *h) { return dg_col_mt_eff(h) * 64 + col_segk(h); }
 
 // the work list of one case: (case c, tile, field, 0) per item
 static void case_work(const dg_handle *h, int c, int mt, std::vector<int4> &work) {
@@ -664,7 +622,7 @@ static int col_tables(dg_handle *h, int mt) {
     return DG_ERR_ARG;
   }
   ColCase cc;
-  DG_TRY(fill_case(h, mt, &cc));
+  fill_case(h, &cc);
   std::vector<int4> work;
   case_work(h, 0, mt, work);
   DG_CUDA(cudaStreamSynchronize(h->st));
@@ -686,17 +644,16 @@ static int col_tables(dg_handle *h, int mt) {
 static int launch_col(cudaStream_t st, int pdl, const dg_col_launch &cl, const void *dev_cases,
                       const int4 *dev_work, int rk_step, long spin, unsigned extra_tx) {
   ColLaunch P;
-  P.tile = cl.tile;
   P.lp = cl.lp;
-  P.nseg = cl.nseg;
   P.nwork = cl.nwork;
-#define CS_CASE(MTV)                                                                            \
-  if (cl.mt == MTV) {                                                                           \
-    dg_big_smem((const void *)k_col_cn<MTV>);                                                   \
-    DG_CUDA(dg_launch(pdl, k_col_cn<MTV>, dim3(cl.grid), dim3(cl.thr), cl.smem, st,             \
+#define CS_CASE(MTV, KV)                                                                        \
+  if (cl.mt == MTV && cl.segk == KV) {                                                          \
+    dg_big_smem((const void *)k_col_cn<MTV, KV>);                                               \
+    DG_CUDA(dg_launch(pdl, k_col_cn<MTV, KV>, dim3(cl.grid), dim3(cl.thr), cl.smem, st,         \
                       (const ColCase *)dev_cases, dev_work, P, rk_step, spin, extra_tx));       \
   }
-  CS_CASE(2) CS_CASE(4) CS_CASE(8) CS_CASE(16)
+  CS_CASE(2, SEG_K) CS_CASE(4, SEG_K) CS_CASE(8, SEG_K) CS_CASE(16, SEG_K)
+  CS_CASE(2, SEG_KS) CS_CASE(4, SEG_KS) CS_CASE(8, SEG_KS) CS_CASE(16, SEG_KS)
 #undef CS_CASE
   DG_LAUNCHED();
   return DG_OK;
@@ -709,22 +666,22 @@ static int col_plan(dg_handle *const *hs, int n, int want, int nwork, dg_col_lau
   for (int c = 0; c < n; c++) mt = std::min(mt, col_mt(hs[c], want));
   dg_col_launch r = {};
   r.mt = mt;
+  r.segk = col_segk(hs[0]);
   for (int c = 0; c < n; c++) {
+    if (col_segk(hs[c]) != r.segk) {
+      dg_set_error("column kernel: columns with different segments cannot share a launch");
+      return DG_ERR_ARG;
+    }
     DG_TRY(col_fits(hs[c], mt));
-    const ColLaunch P = col_sizes(hs[c], mt);
-    r.tile = std::max(r.tile, P.tile);
-    r.lp = std::max(r.lp, P.lp);
-    r.nseg = std::max(r.nseg, P.nseg);
+    r.lp = std::max(r.lp, col_sizes(hs[c]).lp);
     r.thr = std::max(r.thr, col_threads(hs[c], mt));
   }
   ColLaunch P;
-  P.tile = r.tile;
   P.lp = r.lp;
-  P.nseg = r.nseg;
   P.nwork = nwork;
-  r.smem = col_smem_l(P, mt);
+  r.smem = col_smem_l(P, mt, r.thr);
   if (r.smem > 220 * 1024) {
-    dg_set_error("column kernel: the cases' tiles do not fit in shared memory together");
+    dg_set_error("column kernel: the cases' tables do not fit in shared memory");
     return DG_ERR_DIMS;
   }
   r.nwork = nwork;
@@ -775,7 +732,7 @@ int dg_col_batch_build(dg_handle *const *hs, int n, int want_mt, std::vector<uns
   work.clear();
   for (int c = 0; c < n; c++) {
     ColCase cc;
-    DG_TRY(fill_case(hs[c], mt, &cc));
+    fill_case(hs[c], &cc);
     memcpy(cases.data() + sizeof(ColCase) * c, &cc, sizeof(ColCase));
     case_work(hs[c], c, mt, work);
   }

@@ -1,7 +1,6 @@
 // Internal declarations shared by the diablo_b200 CUDA sources.
 #pragma once
 
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string>
@@ -178,6 +177,7 @@ struct dg_handle {
 };
 
 int dg_default_col_mt(const dg_handle *h);
+int dg_default_cn_mt(const dg_handle *h);
 bool dg_mixed_ok(int nx, int nz, int n_th);
 bool dg_per_mixed_ok(int nx, int n_th);
 
@@ -256,10 +256,12 @@ int dg_col_step_dev(dg_handle *h, int rk_step, bool rd);
 size_t dg_col_smem(const dg_handle *h, int mt);
 bool dg_col_th_to_rhs(const dg_handle *h, int n);
 int dg_col_mt_eff(const dg_handle *h);  // modes per CTA the column kernel runs h with
+int dg_col_class(const dg_handle *h);   // cases of one class may share a column launch
 // launch sizes of a column-kernel launch (one case or a server group)
 struct dg_col_launch {
   int mt, thr, grid;      // modes per item, threads per CTA, CTAs (one per item)
-  int tile, lp, nseg;     // shared-memory layout: the largest case's
+  int segk;               // rows per segment (the same for every case)
+  int lp;                 // shared-memory layout: the largest case's table rows
   int nwork;              // work items
   size_t smem;
 };
@@ -286,8 +288,8 @@ static inline int dg_cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 // trigger at kernel entry measured slower: the waiting CTAs held SM slots).
 // dg_pdl_wait() is a no-op for a plain launch.
 __device__ __forceinline__ void dg_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// ------------------------------------------------------------------- TMA
-// Bulk tensor copies (cp.async.bulk.tensor, no multicast) into shared memory,
+// ------------------------------------------------------------ bulk copies
+// Bulk copies (cp.async.bulk, no multicast) into shared memory,
 // completed on an mbarrier.  Waits are bounded: a copy that does not land
 // within the kernel's poll limit (DG_ASYNC_SPIN unless the handle's wait test
 // lowers it for one launch) sets dg_handle::dflag[1] (reported by the next
@@ -307,15 +309,6 @@ __device__ __forceinline__ void dg_mbar_expect_tx(unsigned long long *bar, unsig
                "r"(bytes)
                : "memory");
 }
-// 2-D tiled load of box (x, y) of the tensor map into shared memory at dst
-__device__ __forceinline__ void dg_tma_load_2d(void *dst, const CUtensorMap *map, int x, int y,
-                                               unsigned long long *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(dg_smem_addr(dst)),
-      "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(dg_smem_addr(bar))
-      : "memory");
-}
 // 1-D bulk copy (no multicast) of `bytes` from global to shared memory:
 // both addresses 16-byte aligned, bytes a multiple of 16
 __device__ __forceinline__ void dg_bulk_load(void *dst, const void *src, unsigned bytes,
@@ -325,11 +318,6 @@ __device__ __forceinline__ void dg_bulk_load(void *dst, const void *src, unsigne
           dg_smem_addr(dst)),
       "l"(reinterpret_cast<unsigned long long>(src)), "r"(bytes), "r"(dg_smem_addr(bar))
       : "memory");
-}
-// orders this thread's generic-proxy shared-memory accesses before later
-// bulk copies (async proxy) into the same shared memory
-__device__ __forceinline__ void dg_fence_proxy_async() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 // Folds v >= 0 (or +inf) into the running minimum at *out (the IEEE bit
 // patterns of non-negative doubles order like unsigned integers).  The atomic
@@ -354,10 +342,6 @@ __device__ __forceinline__ bool dg_mbar_wait(unsigned long long *bar, unsigned p
   }
   return false;
 }
-
-// host: a 2-D FP64 tensor map over planes of complex modes -- x = 2*ss
-// doubles of a plane (row stride ss complex), y = rows planes; box 2*mt x by
-int dg_tmap_planes(const void *base, long ss, int rows, int mt, int by, CUtensorMap *out);
 
 template <typename... KArgs, typename... Args>
 static inline cudaError_t dg_launch(int pdl, void (*kern)(KArgs...), dim3 grid, dim3 block,

@@ -95,6 +95,7 @@ struct Group {
   std::vector<cudaEvent_t> ev_m;   // one per member: joins into gs
   cudaEvent_t ev_col = nullptr;    // column launch done: members fork from it
   int cmt = 0;                     // the members' modes per column CTA (all the same)
+  int cls = 0;                     // and their class (dg_col_class)
   void *d_cases = nullptr;         // the column kernel's case table
   int4 *d_work = nullptr;          // and its work list
   dg_col_launch cl = {};           // the column launch's sizes
@@ -452,11 +453,11 @@ struct GroupedLoop {
     }
     // a group's members share one column launch, so they share its modes per
     // CTA: the width each one runs alone (same kernel instance, same results)
-    const int cmt = dg_col_mt_eff(a->h);
+    const int cmt = dg_col_mt_eff(a->h), cls = dg_col_class(a->h);
     Group *best = nullptr;
     double bd = 1e30;
     for (auto &g : groups) {
-      if ((int)(g->m.size() + g->joining.size()) >= s->group_cases || g->cmt != cmt) continue;
+      if ((int)(g->m.size() + g->joining.size()) >= s->group_cases || g->cls != cls) continue;
       const double d = fabs(log(pts(a) / g->points));
       if (d < log(4.0) && d < bd) {
         bd = d;
@@ -466,6 +467,7 @@ struct GroupedLoop {
     if (!best) {
       best = new_group();
       best->cmt = cmt;
+      best->cls = cls;
     }
     best->joining.push_back(a);
     double sum = 0;

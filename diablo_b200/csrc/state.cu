@@ -251,7 +251,7 @@ extern "C" int diablo_gpu_init(const dg_params *p, const double *gy, void *strea
   h->nspec = h->ss * h->nplanes;
   h->nf = 3 + h->NTH;
   h->col_mt = dg_default_col_mt(h);
-  h->cn_mt = 4;
+  h->cn_mt = dg_default_cn_mt(h);
   h->zf_nlo = 1;
   h->pdl = 1;
   h->plane_xz = 1;
@@ -449,7 +449,7 @@ extern "C" int diablo_gpu_finalize(dg_handle *h) {
   return DG_OK;
 }
 
-// dflag[1] is set by a kernel whose bulk tensor copies did not land within
+// dflag[1] is set by a kernel whose bulk copies did not land within
 // its bounded wait (the kernel then skipped its work).  Reported once: the
 // flag is cleared, so the next call reports only a new failure.
 static int check_async_flag(dg_handle *h) {
@@ -459,7 +459,7 @@ static int check_async_flag(dg_handle *h) {
   if (f) {
     DG_CUDA(cudaMemsetAsync(h->dflag + 1, 0, sizeof(int), h->st));
     DG_CUDA(cudaStreamSynchronize(h->st));
-    dg_set_error("a bulk tensor copy did not complete within its wait limit; the substep's "
+    dg_set_error("a bulk copy did not complete within its wait limit; the substep's "
                  "results are invalid");
     return DG_ERR_TIMEOUT;
   }

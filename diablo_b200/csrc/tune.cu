@@ -89,6 +89,13 @@ int dg_default_col_mt(const dg_handle *h) {
   return 4;
 }
 
+// 8 modes fill whole 128-byte lines of a row (40.8 us per launch at
+// Re_tau = 180, 44.4 with 4, 44 with 16; 1107 us at 512x257x384, 1151 with 4);
+// 4 where 8 would leave SMs without a CTA
+int dg_default_cn_mt(const dg_handle *h) {
+  return (long)h->nf * ((h->ss + 7) / 8) < 148 ? 4 : 8;
+}
+
 static void invalidate_graphs(dg_handle *h) {
   dg_graphs_free(h);
   h->gwarm[0] = h->gwarm[1] = false;
