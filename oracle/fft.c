@@ -20,7 +20,7 @@
 #include <string.h>
 #include "oracle_int.h"
 
-#define MAX_PLANS 16
+#define MAX_PLANS 64  /* transform lengths of one process */
 
 typedef struct {
   int n;
