@@ -947,8 +947,7 @@ size_t zw_smem(int nz) {
   return sizeof(CX) * (nz + 4 * 2 * zw_kpw(nz) * (size_t)padded_len(nz));
 }
 
-// NLO as for k_zfwd_rhs: only -i kz A + B goes out, into rhs.
-template <int NZ, typename CX = double2, bool NLO = false, int PV = 0>
+template <int NZ, typename CX = double2, int PV = 0>
 __global__ void __launch_bounds__(128, zw_minb(NZ, sizeof(CX))) k_zfwd_w(
     ChanConst C, const CX *__restrict__ G, long Gfield, const CX *__restrict__ tw,
     const double *__restrict__ dscal, int rk_step, const double *__restrict__ kxv,
@@ -1027,10 +1026,6 @@ __global__ void __launch_bounds__(128, zw_minb(NZ, sizeof(CX))) k_zfwd_w(
     const double KX = kxv[kx], KZ = kzv[kp];
     const double2 nlv = make_double2(KZ * a.y + b.x, -KZ * a.x + b.y);  // -i kz A + B
     const long o = (long)j * ss + (long)kp * nkxp + kx;
-    if constexpr (NLO) {
-      rhs(f)[o] = nlv;
-      continue;
-    }
     const double k2 = KX * KX + KZ * KZ;
     const double kk = (C.beta == 1.0) ? k2 : pow(k2, C.beta);
     const bool mean = (kx == 0 && kp == 0);
@@ -1132,11 +1127,11 @@ __global__ void __launch_bounds__(128, zw_minb(NZ, sizeof(CX))) k_zfwd_w(
   }
 }
 
-template <int NZ, typename CX, bool NLO>
+template <int NZ, typename CX>
 auto zfwd_kernel(int v) {
   if constexpr (plan_has_variant(NZ))
-    if (v) return k_zfwd_w<NZ, CX, NLO, 1>;
-  return k_zfwd_w<NZ, CX, NLO, 0>;
+    if (v) return k_zfwd_w<NZ, CX, 1>;
+  return k_zfwd_w<NZ, CX, 0>;
 }
 
 __host__ __device__ constexpr bool zw_supported(int n) {
@@ -1983,7 +1978,7 @@ int dg_courant_dev(dg_handle *h, const double2 *const *u, bool side) {
   }
   auto run = [&]() -> int {
     h->pdl_zinv = 0;
-    DG_TRY(dg_zinv(h, u, 3, 1, h->NY, h->H, 0));
+    DG_TRY(dg_zinv(h, u, 3, 1, h->NY, h->H, false));
     DG_CUDA(cudaMemsetAsync(h->dmin_bits, 0x7f, sizeof(unsigned long long), h->st));
     DG_TRY(dg_xc2r_cfl(h, h->H, 1, h->NY, h->dmin_bits));
     dg_kt_begin(h, "k_dt_update", h->st);
@@ -2089,13 +2084,13 @@ static int nl_chunk_mixed(dg_handle *h, const ChanConst &C, int rk_step, int a, 
     return DG_ERR_DIMS;
   }
   DG_LAUNCHED();
+  if (h->zf_nlo) return dg_cols_nl(h, a, b);
   dim3 zgrid(dg_cdiv(h->nkxp, zw_kxg(h->NZ)), nplan, h->nf);
   const size_t sm = zw_smem<float2>(h->NZ);
   done = false;
 #define ZW_CASE(N)                                                                              \
   if (!done && h->NZ == N) {                                                                    \
-    auto kern = h->zf_nlo ? zfwd_kernel<N, float2, true>(h->fft_plan)                           \
-                          : zfwd_kernel<N, float2, false>(h->fft_plan);                         \
+    auto kern = zfwd_kernel<N, float2>(h->fft_plan);                                            \
     dg_big_smem((const void *)kern);                                                            \
     dg_kt_begin(h, "k_zfwd_w_f32", h->st);                                                      \
     DG_CUDA(dg_launch(h->pdl, kern, zgrid, dim3(128), sm, h->st, C, Gf, Hfield,                 \
@@ -2173,13 +2168,13 @@ static int nl_generic_mixed(dg_handle *h, const ChanConst &C, int rk_step,
     }
     DG_LAUNCHED();
   }
+  if (h->zf_nlo) return dg_cols_nl(h, 1, NY);
   done = false;
   dim3 zgrid(dg_cdiv(h->nkxp, zw_kxg(NZ)), NY, h->nf);
   const size_t sm = zw_smem<float2>(NZ);
 #define ZW_CASE(N)                                                                              \
   if (!done && NZ == N) {                                                                       \
-    auto kern = h->zf_nlo ? zfwd_kernel<N, float2, true>(h->fft_plan)                           \
-                          : zfwd_kernel<N, float2, false>(h->fft_plan);                         \
+    auto kern = zfwd_kernel<N, float2>(h->fft_plan);                                            \
     dg_big_smem((const void *)kern);                                                            \
     dg_kt_begin(h, "k_zfwd_w_f32", h->st);                                                      \
     DG_CUDA(dg_launch(h->pdl, kern, zgrid, dim3(128), sm, h->st, C, Gf, Hfield,                 \
@@ -2238,7 +2233,7 @@ int dg_chan_nonlinear(dg_handle *h, int time_step, int rk_step, bool *column_nex
     }
     // 1. z inverse of the planes this chunk's x-rows need (a-1 .. b+1)
     h->pdl_zinv = h->pdl;
-    const int zs = dg_zinv(h, in, h->nf, hdone + 1, b + 1, h->H, 0);
+    const int zs = dg_zinv(h, in, h->nf, hdone + 1, b + 1, h->H, false);
     h->pdl_zinv = 0;
     DG_TRY(zs);
     hdone = b + 1;
@@ -2272,7 +2267,7 @@ int dg_chan_nonlinear(dg_handle *h, int time_step, int rk_step, bool *column_nex
     if (!done) {
       // generic CTA kernel covers all planes 1..NY in one launch
       if (a == 1) {
-        DG_TRY(dg_zinv(h, in, h->nf, hdone + 1, h->NY + 1, h->H, 0));
+        DG_TRY(dg_zinv(h, in, h->nf, hdone + 1, h->NY + 1, h->H, false));
         hdone = h->NY + 1;
         if (dg_xmarch_ok(h)) {
           DG_TRY(dg_xmarch(h));
@@ -2303,13 +2298,19 @@ int dg_chan_nonlinear(dg_handle *h, int time_step, int rk_step, bool *column_nex
     //    planes 1..NY after the generic x-row stage)
     const int za = done ? a : 1, zb = done ? b : h->NY;
     bool zdone = false;
-    if (zw_supported(h->NZ) || zw_big(h->NZ)) {
+    if (h->zf_nlo) {
+      const int zs = dg_cols_nl(h, za, zb);
+      if (zs != 1) {
+        DG_TRY(zs);
+        zdone = true;
+      }
+    }
+    if (!zdone && (zw_supported(h->NZ) || zw_big(h->NZ))) {
       dim3 grid(dg_cdiv(h->nkxp, zw_kxg(h->NZ)), zb - za + 1, h->nf);
       const size_t sm = zw_smem<double2>(h->NZ);
 #define ZW_CASE(N)                                                                             \
   if (h->NZ == N) {                                                                            \
-    auto kern = h->zf_nlo ? zfwd_kernel<N, double2, true>(h->fft_plan)                         \
-                          : zfwd_kernel<N, double2, false>(h->fft_plan);                       \
+    auto kern = zfwd_kernel<N, double2>(h->fft_plan);                                          \
     dg_big_smem((const void *)kern);                                                           \
     dg_kt_begin(h, "k_zfwd_w", h->st);                                                          \
     DG_CUDA(dg_launch(h->pdl, kern, grid, dim3(128), sm, h->st, C, h->G, Hfield, h->twz,       \
@@ -2325,19 +2326,12 @@ int dg_chan_nonlinear(dg_handle *h, int time_step, int rk_step, bool *column_nex
     if (!zdone && (!done || b == h->NY)) {
       dim3 grid(dg_cdiv(h->nkxp, zf_kxg(h->NZ)), h->NY);
       const size_t sm = zfwd_smem(h);
-#define KERNEL_BODY(N)                                                                          \
-  {                                                                                             \
-    auto kern = h->zf_nlo ? k_zfwd_rhs<N, true> : k_zfwd_rhs<N, false>;                         \
-    dg_big_smem((const void *)kern);                                                            \
-    dg_kt_begin(h, "k_zfwd_rhs", h->st);                                                        \
-    kern<<<grid, ZF_THR, sm, h->st>>>(C, h->G, Hfield, h->plz, h->twz, h->dscal, rk_step,       \
-                                      h->kx, h->kz, h->dy, h->dyf, cu, cf, rhs, h->cp);         \
-  }
-      switch (h->NZ) {
-        DG_FOR_EACH_N(DG_CASE_N)
-        default: KERNEL_BODY(0); break;
-      }
-#undef KERNEL_BODY
+      // (compile-time lengths take one of the two above)
+      auto kern = h->zf_nlo ? k_zfwd_rhs<0, true> : k_zfwd_rhs<0, false>;
+      dg_big_smem((const void *)kern);
+      dg_kt_begin(h, "k_zfwd_rhs", h->st);
+      kern<<<grid, ZF_THR, sm, h->st>>>(C, h->G, Hfield, h->plz, h->twz, h->dscal, rk_step, h->kx,
+                                        h->kz, h->dy, h->dyf, cu, cf, rhs, h->cp);
       DG_LAUNCHED();
     }
     if (!done) break;  // the generic kernels covered every plane
@@ -2475,7 +2469,7 @@ int dg_stats_dev(dg_handle *h, dg_stats *s) {
       NY, h->ss, h->nkxp, h->kx, h->kz, h->dyf, h->cu[0], h->cu[1], h->cu[2], dspec);
   DG_LAUNCHED();
   const double2 *dd[1] = {dspec};
-  DG_TRY(dg_zinv(h, dd, 1, 2, NY - 1, h->H, 0));
+  DG_TRY(dg_zinv(h, dd, 1, 2, NY - 1, h->H, false));
   const long pplane = (long)h->NZ * h->NX;
   double *phys = (double *)h->work;
   DG_TRY(dg_xc2r_planes(h, h->H, 1, 2, NY - 1, phys - 2 * pplane, pplane, h->NX, 0));

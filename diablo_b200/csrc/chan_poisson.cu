@@ -135,7 +135,7 @@ extern "C" int diablo_poisson_p_chan(dg_handle *h) {
     DG_LAUNCHED();
     const int nf = (stage == 0) ? 3 : 2;
     const double2 *in[3] = {s[0], s[1], s[2]};
-    DG_TRY(dg_zinv(h, in, nf, 2, NY, h->H, 0));
+    DG_TRY(dg_zinv(h, in, nf, 2, NY, h->H, false));
     // stage 0 fills W0..W2, later stages W1..W2
     double *dst = (stage == 0) ? W : W + pfield;
     DG_TRY(dg_xc2r_planes(h, h->H, nf, 2, NY, dst, pplane, h->NX, pfield));
@@ -146,7 +146,7 @@ extern "C" int diablo_poisson_p_chan(dg_handle *h) {
   }
   DG_TRY(dg_xr2c_planes(h, W, 1, 2, NY, pplane, h->NX, 0, h->H));
   double2 *out[1] = {s[0]};
-  DG_TRY(dg_zfwd_planes(h, h->H, 1, 2, NY, out, nullptr, 0));
+  DG_TRY(dg_zfwd_planes(h, h->H, 1, 2, NY, out, false));
   CFieldPtrs th;
   for (int n = 0; n < h->NTH; n++) th.p[n] = h->cu[3 + n];
   RiVals ri;

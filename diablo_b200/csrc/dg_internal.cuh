@@ -210,15 +210,31 @@ int dg_cfwd_ff(dg_handle *h, const float2 *H, long in_field, int nf, int jmin, i
 int dg_cfwd_g(dg_handle *h, const double2 *H, long in_field, int nf, int jmin, int jmax,
               int rowlen, int nkt, int N, int NK, const FftPlan &pl, const double2 *tw,
               double2 *const *fields, long out_plane);
+// the same transforms with one exchange through shared memory (fft_cols.cu);
+// 1 where the length has no such split
+int dg_cols_inv(dg_handle *h, const double2 *const *f, int nf, int jmin, int jmax, long in_plane,
+                int rowlen, int n, int nk, const double2 *tw, double2 *H, long out_field);
+int dg_cols_inv(dg_handle *h, const double2 *const *f, int nf, int jmin, int jmax, long in_plane,
+                int rowlen, int n, int nk, const float2 *tw, float2 *H, long out_field);
+int dg_cols_inv(dg_handle *h, const float2 *const *f, int nf, int jmin, int jmax, long in_plane,
+                int rowlen, int n, int nk, const float2 *tw, float2 *H, long out_field);
+int dg_cols_fwd(dg_handle *h, const double2 *H, long in_field, int nf, int jmin, int jmax,
+                int rowlen, int n, int nk, const double2 *tw, double2 *const *f, long out_plane);
+int dg_cols_fwd(dg_handle *h, const float2 *H, long in_field, int nf, int jmin, int jmax,
+                int rowlen, int n, int nk, const float2 *tw, float2 *const *f, long out_plane);
+// G of planes jmin..jmax to the nonlinear terms -i kz A + B in the rhs arrays
+int dg_cols_nl(dg_handle *h, int jmin, int jmax);
+// plane_form: the passes of the whole-plane kernels (dg_plane_c2r, dg_plane_r2c), where
+// they exist for the lengths, so that the staged pair gives the same bits
 int dg_zinv(dg_handle *h, const double2 *const *fields, int nf, int jmin, int jmax,
-            double2 *H, int field_stride_planes);
+            double2 *H, bool plane_form);
 int dg_xc2r_planes(dg_handle *h, const double2 *H, int nf, int jmin, int jmax, double *phys,
                    long phys_plane_stride, long phys_row_stride, long field_stride);
 int dg_xc2r_cfl(dg_handle *h, const double2 *H, int jmin, int jmax, unsigned long long *out);
 int dg_xr2c_planes(dg_handle *h, const double *phys, int nf, int jmin, int jmax,
                    long phys_plane_stride, long phys_row_stride, long field_stride, double2 *H);
 int dg_zfwd_planes(dg_handle *h, const double2 *H, int nf, int jmin, int jmax,
-                   double2 *const *fields, double2 *raw_ref, long raw_ld);
+                   double2 *const *fields, bool plane_form);
 // whole-plane transforms (spectral planes <-> physical rows, one kernel per
 // direction, no staging array): DG_OK once launched, 1 when the grid does not
 // allow them (the caller then stages through a half-physical array)

@@ -538,6 +538,10 @@ auto xc2r_cfl_kernel(int v) {
 
 // ------------------------------------------------------------- host wrappers
 
+// Lengths of the whole-plane kernels: x and z lengths with a compile-time
+// warp plan up to 128 (the z columns of a plane then fit two CTAs per SM).
+#define DG_PLANE_NX(X) X(16) X(32) X(48) X(64) X(96) X(128)
+
 // Column transforms along one axis for a batch of planes.  Geometry (per
 // field): input plane j at fields[f] + j*in_plane, packed slot kp of column c
 // at + kp*rowlen + c; output plane j at H + f*out_field + j*N*rowlen, bin z of
@@ -546,9 +550,13 @@ auto xc2r_cfl_kernel(int v) {
 template <typename CI, typename CX>
 static int cinv_t(dg_handle *h, const CI *const *fields, int nf, int jmin, int jmax,
                   long in_plane, int rowlen, int N, int NK, const FftPlan &pl, const CX *tw, CX *H,
-                  long out_field) {
+                  long out_field, bool plane_form = false) {
   using PA = PtrArray<const CI>;
   if (jmax < jmin || nf <= 0) return DG_OK;
+  if (!plane_form) {
+    const int s = dg_cols_inv(h, fields, nf, jmin, jmax, in_plane, rowlen, N, NK, tw, H, out_field);
+    if (s != 1) return s;
+  }
   PA fp;
   for (int f = 0; f < nf; f++) fp.p[f] = fields[f];
   dim3 grid(dg_cdiv(rowlen, batch_for(N)), jmax - jmin + 1, nf);
@@ -561,9 +569,14 @@ static int cinv_t(dg_handle *h, const CI *const *fields, int nf, int jmin, int j
     DG_CUDA(dg_launch(h->pdl_zinv, kern, grid, dim3(NTHR), sm, h->st, fp, jmin, in_plane,     \
                       rowlen, N, NK, pl, tw, H, out_field));                                  \
   }
-  switch (N) {
-    DG_FOR_EACH_N(DG_CASE_N)
-    default: KERNEL_BODY(0); break;
+  // compile-time lengths: the plane form's only (dg_cols_inv takes the others)
+  if constexpr (std::is_same<CI, double2>::value && std::is_same<CX, double2>::value) {
+    switch (N) {
+      DG_PLANE_NX(DG_CASE_N)
+      default: KERNEL_BODY(0); break;
+    }
+  } else {
+    KERNEL_BODY(0);
   }
 #undef KERNEL_BODY
   DG_LAUNCHED();
@@ -591,8 +604,12 @@ int dg_cinv_ff(dg_handle *h, const float2 *const *fields, int nf, int jmin, int 
 template <typename CX, typename PO, typename OUT>
 static int cfwd_t(dg_handle *h, const CX *H, long in_field, int nf, int jmin, int jmax, int rowlen,
                   int nkt, int N, int NK, const FftPlan &pl, const CX *tw, OUT *const *fields,
-                  long out_plane) {
+                  long out_plane, bool plane_form = false) {
   if (jmax < jmin || nf <= 0) return DG_OK;
+  if (!plane_form) {
+    const int s = dg_cols_fwd(h, H, in_field, nf, jmin, jmax, rowlen, N, NK, tw, fields, out_plane);
+    if (s != 1) return s;
+  }
   PO fp;
   for (int f = 0; f < nf; f++) fp.p[f] = fields[f];
   dim3 grid(dg_cdiv(rowlen, batch_for(N)), jmax - jmin + 1, nf);
@@ -602,9 +619,13 @@ static int cfwd_t(dg_handle *h, const CX *H, long in_field, int nf, int jmin, in
   dg_kt_begin(h, "k_zfwd", h->st);                                                             \
   k_zfwd<NN, CX, PO><<<grid, NTHR, sm, h->st>>>(H, in_field, jmin, rowlen, nkt, N, NK, pl, tw, fp, \
                                                out_plane)
-  switch (N) {
-    DG_FOR_EACH_N(DG_CASE_N)
-    default: KERNEL_BODY(0); break;
+  if constexpr (std::is_same<CX, double2>::value) {
+    switch (N) {
+      DG_PLANE_NX(DG_CASE_N)
+      default: KERNEL_BODY(0); break;
+    }
+  } else {
+    KERNEL_BODY(0);
   }
 #undef KERNEL_BODY
   DG_LAUNCHED();
@@ -625,16 +646,20 @@ int dg_cfwd_ff(dg_handle *h, const float2 *H, long in_field, int nf, int jmin, i
                                           tw, fields, out_plane);
 }
 
+// the whole-plane kernels exist for the handle's lengths
+static bool plane_lengths(const dg_handle *h);
+
 int dg_zinv(dg_handle *h, const double2 *const *fields, int nf, int jmin, int jmax, double2 *H,
-            int) {
-  return dg_cinv_g(h, fields, nf, jmin, jmax, h->ss, h->nkxp, h->NZ, h->NKZ, h->plz, h->twz, H,
-                   (long)h->nplanes * h->NZ * h->nkxp);
+            bool plane_form) {
+  return cinv_t(h, fields, nf, jmin, jmax, h->ss, h->nkxp, h->NZ, h->NKZ, h->plz, h->twz, H,
+                (long)h->nplanes * h->NZ * h->nkxp, plane_form && plane_lengths(h));
 }
 
 int dg_zfwd_planes(dg_handle *h, const double2 *H, int nf, int jmin, int jmax,
-                   double2 *const *fields, double2 *, long) {
-  return dg_cfwd_g(h, H, (long)h->nplanes * h->NZ * h->nkxp, nf, jmin, jmax, h->nkxp, h->nkzt,
-                   h->NZ, h->NKZ, h->plz, h->twz, fields, h->ss);
+                   double2 *const *fields, bool plane_form) {
+  return cfwd_t<double2, FieldPtrs>(h, H, (long)h->nplanes * h->NZ * h->nkxp, nf, jmin, jmax,
+                                    h->nkxp, h->nkzt, h->NZ, h->NKZ, h->plz, h->twz, fields, h->ss,
+                                    plane_form && plane_lengths(h));
 }
 
 int dg_xc2r_planes(dg_handle *h, const double2 *H, int nf, int jmin, int jmax, double *phys,
@@ -678,18 +703,15 @@ int dg_xr2c_planes(dg_handle *h, const double *phys, int nf, int jmin, int jmax,
 }
 
 // ------------------------------------------------- whole-plane transforms
-// Lengths of the whole-plane kernels: x and z lengths with a compile-time
-// warp plan up to 128 (the z columns of a plane then fit two CTAs per SM).
-#define DG_PLANE_NX(X) X(16) X(32) X(48) X(64) X(96) X(128)
-
-bool dg_plane_ok(const dg_handle *h) {
+static bool plane_lengths(const dg_handle *h) {
   auto len_ok = [](int n) {
     return n == 16 || n == 32 || n == 48 || n == 64 || n == 96 || n == 128;
   };
-  return h->plane_xz && !h->periodic && len_ok(h->NX) && len_ok(h->NZ) &&
-         h->nkxp == h->NX / 3 + 1 && h->NKZ == h->NZ / 3 &&
-         h->ss == (long)h->nkxp * (2 * h->NKZ + 1);
+  return !h->periodic && len_ok(h->NX) && len_ok(h->NZ) && h->nkxp == h->NX / 3 + 1 &&
+         h->NKZ == h->NZ / 3 && h->ss == (long)h->nkxp * (2 * h->NKZ + 1);
 }
+
+bool dg_plane_ok(const dg_handle *h) { return h->plane_xz && plane_lengths(h); }
 
 namespace {
 // the whole-plane kernels run two CTAs per SM at the largest sizes only with

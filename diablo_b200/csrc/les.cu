@@ -630,7 +630,7 @@ int to_physical(dg_handle *h, const double2 *const *in, int n, int jmin, int jma
       DG_TRY(r);
       continue;
     }
-    DG_TRY(dg_zinv(h, in + b, k, jmin, jmax, h->les_H, 0));
+    DG_TRY(dg_zinv(h, in + b, k, jmin, jmax, h->les_H, true));
     DG_TRY(dg_xc2r_planes(h, h->les_H, k, jmin, jmax, out + (long)b * pf, pplane, h->NX, pf));
   }
   return DG_OK;
@@ -646,7 +646,7 @@ int to_fourier(dg_handle *h, const double *in, int n, int jmin, int jmax, double
       continue;
     }
     DG_TRY(dg_xr2c_planes(h, in + (long)b * pf, k, jmin, jmax, pplane, h->NX, pf, h->les_H));
-    DG_TRY(dg_zfwd_planes(h, h->les_H, k, jmin, jmax, out + b, nullptr, 0));
+    DG_TRY(dg_zfwd_planes(h, h->les_H, k, jmin, jmax, out + b, true));
   }
   return DG_OK;
 }

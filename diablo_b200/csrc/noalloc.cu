@@ -235,7 +235,7 @@ extern "C" int diablo_fft_xz_to_fourier_noalloc(const double *V, double *VV, int
     const int nj = (jmax - j0 + 1 < chunk) ? jmax - j0 + 1 : chunk;
     DG_TRY(dg_xr2c_planes(&hh, V + (long)j0 * pplane, 1, 0, nj - 1, pplane, nx + 2, 0, H));
     double2 *flds[1] = {cmp};
-    DG_TRY(dg_zfwd_planes(&hh, H, 1, 0, nj - 1, flds, nullptr, 0));
+    DG_TRY(dg_zfwd_planes(&hh, H, 1, 0, nj - 1, flds, false));
     k_na_expand<<<dg_cdiv((long)nj * nz2 * nxp1, 256), 256, 0, hh.st>>>(
         cmp, (double2 *)(VV + (long)j0 * pplane), nj, nkzt, nkxp, nxp1, nz2);
     DG_LAUNCHED();

@@ -105,7 +105,7 @@ extern "C" int diablo_fft_xz_to_fourier(dg_handle *h, const double *V, double *V
   DG_TRY(dg_xr2c_planes(h, vin - (long)jmin * pplane, 1, jmin, jmax, pplane, h->NX + 2, 0, h->H));
   double2 *cmp = h->rhs[0];
   double2 *flds[1] = {cmp};
-  DG_TRY(dg_zfwd_planes(h, h->H, 1, jmin, jmax, flds, nullptr, 0));
+  DG_TRY(dg_zfwd_planes(h, h->H, 1, jmin, jmax, flds, false));
   double2 *dref = (double2 *)(where == DG_HOST ? tin : vout);
   k_compact_to_ref_planes<<<dg_cdiv((long)nj * nz2 * nxp1, 256), 256, 0, h->st>>>(
       cmp + (long)jmin * h->ss, dref, nj, h->nkzt, h->nkxp, nxp1, nz2);
@@ -143,7 +143,7 @@ extern "C" int diablo_fft_xz_to_physical(dg_handle *h, const double *VV, double 
       (const double2 *)sin_, cmp + (long)jmin * h->ss, nj, h->nkzt, h->nkxp, nxp1, nz2);
   DG_LAUNCHED();
   const double2 *flds[1] = {cmp};
-  DG_TRY(dg_zinv(h, flds, 1, jmin, jmax, h->H, 0));
+  DG_TRY(dg_zinv(h, flds, 1, jmin, jmax, h->H, false));
   DG_TRY(dg_xc2r_planes(h, h->H, 1, jmin, jmax, pout - (long)jmin * pplane, pplane, h->NX + 2, 0));
   if (where == DG_HOST) {
     DG_CUDA(cudaMemcpyAsync(V + (long)jmin * pplane, tout, bytes, cudaMemcpyDeviceToHost, h->st));

@@ -525,3 +525,27 @@ def test_marching_rows_match_oracle(nx, n_th, ny, chunk, precision):
         ch.step(s)
     compare(ref, ch, fields(p), tol=TOL if precision == 0 else 1e-5)
     ch.close()
+
+
+@pytest.mark.parametrize("precision,nx,nz,n_th", [
+    (0, 32, 18, 1), (0, 36, 20, 0), (0, 48, 30, 0), (0, 32, 54, 0), (0, 20, 80, 0), (0, 16, 90, 0),
+    (0, 16, 96, 1), (0, 16, 150, 0), (0, 16, 192, 0), (0, 16, 240, 0), (0, 16, 256, 0),
+    (0, 16, 270, 0), (0, 16, 324, 0), (0, 16, 384, 0), (0, 16, 512, 0), (0, 16, 540, 0),
+    (0, 16, 1024, 0), (1, 32, 48, 1), (1, 32, 192, 0), (1, 16, 256, 0), (1, 16, 384, 0),
+    (1, 16, 512, 0)])
+def test_column_transforms_match_oracle(precision, nx, nz, n_th):
+    """The z transforms in one and two exchanges: every compile-time length,
+    run-time lengths with each radix (2..16) and of every group size, and tiles with a
+    partial last group of columns, over 2 steps against the oracle.
+    FP32: the mixed form's bar."""
+    p, gy = configs.channel_re180(nx=nx, ny=9, nz=nz)
+    p = p.replace(n_th=n_th, precision=precision, variable_dt=1, cfl=0.3, delta_t=2e-4)
+    p.pr = [0.71, 1, 1, 1]
+    p.th_bc_ymin_c1 = [-1.0, 0, 0, 0]
+    p.th_bc_ymax_c1 = [1.0, 0, 0, 0]
+    ref, ch, _ = start_pair(p, gy, ics.channel_laminar, seed=37)
+    for s in (1, 2):
+        ref.step(s)
+        ch.step(s)
+    compare(ref, ch, fields(p), tol=TOL if precision == 0 else 1e-5)
+    ch.close()
