@@ -3,20 +3,22 @@
 //
 // One substep is five launches (plus COURANT's on the side stream when it
 // runs):
-//   zinv        spectral U1..U3, TH -> half-physical H (z inverse per kx)
-//   k_xrow_w    per physical z-row, marching up in y: x c2r of every field,
+//   k_cols_inv  spectral U1..U3, TH -> half-physical H (z inverse per kx;
+//               fft_cols.cu)
+//   k_xrows     per physical z-row, marching up in y: x c2r of every field,
 //               all products/fluxes of for/channel.f:409-571,665-720, x r2c,
 //               and the combination into 2 arrays per field
-//               (A: to be multiplied by -i kz, B: the rest).  Row lengths
-//               without a warp kernel take two launches instead: k_xc2r of
+//               (A: to be multiplied by -i kz, B: the rest); chan_xrows.cu for rows of
+//               16 to 128 points, k_xmarch (chan_xmarch.cu) for 192 to 512.  Other row
+//               lengths and N_TH > 2 take two launches instead: k_xc2r of
 //               every plane into physical space, then k_xprod (products, x
 //               r2c and the combination, one product pair per CTA).
-//   k_zfwd_w    per plane: z forward of A/B -> the nonlinear term
-//               NL = -i kz A + B of every retained mode (with LES, whose
-//               solves need them, the epilogue also forms the explicit terms,
+//   k_cols_nl   per plane: z forward of A/B -> the nonlinear term
+//               NL = -i kz A + B of every retained mode (fft_cols.cu).  With LES, whose
+//               solves need them, k_zfwd_w's epilogue also forms the explicit terms,
 //               CF and the Crank-Nicolson right-hand side
 //               R = CU + zeta h CF_old - h grad P + beta h CF_new
-//                   + (nu h / 2) d2/dy2 CU,          for/channel.f:88-626)
+//                   + (nu h / 2) d2/dy2 CU,          for/channel.f:88-626
 //   k_col_cn    per (mode tile, field) (chan_column.cu): explicit terms, CF,
 //               the CN right-hand side and solve.  The reference solves the
 //               same x-z independent CN operator per physical column
@@ -246,7 +248,7 @@ __global__ void __launch_bounds__(XP_THR, 5) k_xprod(
 
 // ------------------------------------------------- generic x-row stage, FP32
 // The mixed form of the two launches above, for the compile-time row lengths
-// without a warp x-row kernel (and for N_TH > 2).  As in k_xrow_w's FP32
+// where neither k_xrows nor k_xmarch runs (N_TH > 2).  As in their FP32
 // form, every x-row is split into its mean (FP64) and its fluctuation
 // (FP32): k_xc2r_f takes the FP32 half-physical planes to physical
 // fluctuation rows (the kx = 0 bin removed) and keeps each row's mean;
@@ -462,291 +464,6 @@ __global__ void __launch_bounds__(XP_THR) k_xprod_f(
       if (n + 1 < nth) o[(8 + 2 * n) * Gfield] = Bf;
     }
   }
-}
-
-// ------------------------------------------------------- xrow, one warp/row
-// Same products as listed above, organised so a warp owns one physical z-row and
-// marches up through its chunk of planes with no CTA-wide barrier: the two
-// physical planes it needs (j and j+1) live in registers (lane l holds
-// x = l + 32 i), the transforms run in a per-warp shared buffer with
-// __syncwarp between passes, and the x-spectra carried from one plane to the
-// next (fluxes at GY j, Ubar U2 at GY j, g at GYF j-1) live in registers
-// (lane l holds kx = l + 32 s).  At step j it forms the GYF-j products and
-// the GY-(j+1) products, so only planes j and j+1 are needed.
-constexpr int XW_WARPS = 4;
-
-__host__ __device__ constexpr bool xw_supported(int n) {
-  return n == 16 || n == 32 || n == 48 || n == 64 || n == 96 || n == 128 || n == 256;
-}
-
-template <int NX, int NTH, typename CX = double2, int PV = 0>
-__global__ void __launch_bounds__(32 * XW_WARPS, NTH == 0 ? (sizeof(CX) == 8 ? 4 : 3) : 2) k_xrow_w(
-    ChanConst C, const CX *__restrict__ H, long Hfield, int chunk, int jbase, int jtop,
-    const CX *__restrict__ tw, const double *__restrict__ dyf, const double *__restrict__ dy,
-    const double *__restrict__ kxv, CX *__restrict__ G, long Gfield) {
-  constexpr int NF = 3 + NTH;
-  constexpr int NPIN = (NF + 1) / 2;
-  constexpr int NPROD = 8 + 3 * NTH;
-  constexpr int NPP = (NPROD + 1) / 2;
-  constexpr int MAXP = NPIN > NPP ? NPIN : NPP;
-  constexpr int XPL = (NX + 31) / 32;              // physical points per lane
-  constexpr int NKXP = NX / 3 + 1;
-  constexpr int KS = (NKXP + 31) / 32;             // kx slots per lane
-  constexpr int SSTR = padded_len(NX);
-  extern __shared__ double2 sm_raw[];
-  using T = typename CT<CX>::T;
-  CX *sm = reinterpret_cast<CX *>(sm_raw);
-  CX *stw = sm;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  CX *buf = stw + NX + warp * MAXP * SSTR;
-  // carried x-spectra: 0 fl1, 1 fl3, 2 ubar1 u2, 3 ubar3 u2, 4 g, 5+n flth
-  CX *pvs = stw + NX + XW_WARPS * MAXP * SSTR + warp * (5 + NTH) * NKXP;
-  stage_tw<NX, PV, tp_ok(NX)>(stw, tw, NX, threadIdx.x, blockDim.x);
-  dg_pdl_wait();  // H comes from the z inverse
-  __syncthreads();
-  const int z = blockIdx.x * XW_WARPS + warp;
-  const int NZ = C.NZ;
-  if (z >= NZ) return;
-  const int j0 = jbase + blockIdx.y * chunk;
-  int j1 = j0 + chunk - 1;
-  if (j1 > jtop) j1 = jtop;
-  const T rnx = (T)1 / (T)NX;            // exact: NX is 2^a 3^b ... see below
-  const bool pow2 = (NX & (NX - 1)) == 0;
-  const long plane = (long)NZ * NKXP;
-
-  T cur[NF][XPL], nxt[NF][XPL];
-#define PV(q, s) pvs[(q) * NKXP + lane + 32 * (s)]
-
-  // FP32 form: each x-row is split into its x-mean (kept in FP64, uniform
-  // across the row) and the fluctuation (FP32).  The transforms see only
-  // fluctuations, so the two real rows packed into one complex transform
-  // have comparable magnitude, and the row means of the products are formed
-  // in FP64 from the means and the fluctuations.
-  constexpr bool F32 = sizeof(T) == 4;
-  double dcur[NF], dnxt[NF];
-  auto load_plane = [&](int pl, T (&dst)[NF][XPL], double (&dcv)[NF]) {
-    const CX *row = H + (long)pl * plane + (long)z * NKXP;
-    if constexpr (F32) {
-#pragma unroll
-      for (int f = 0; f < NF; f++) dcv[f] = (double)row[f * Hfield].x;
-    }
-#pragma unroll
-    for (int q = 0; q < NPIN; q++) {
-      const int fa = 2 * q, fb = 2 * q + 1;
-#pragma unroll
-      for (int i = 0; i < (NX + 31) / 32; i++) {
-        const int k = lane + 32 * i;
-        const int kk = (k <= NX / 2) ? k : NX - k;
-        // bins above NKX (the truncated band, the x-Nyquist bin among them)
-        // are zero: the pruned first pass below does not read them
-        if (k < NX && kk < NKXP && kk < NX / 2) {
-          CX a = row[fa * Hfield + kk];
-          CX bb = (fb < NF) ? row[fb * Hfield + kk] : CT<CX>::mk(0, 0);
-          if (kk == 0) { a.y = 0.0; bb.y = 0.0; }
-          if (F32 && kk == 0) { a.x = 0.0; bb.x = 0.0; }
-          buf[q * SSTR + pad(k)] = (k == kk) ? CT<CX>::mk(a.x - bb.y, a.y + bb.x)
-                                             : CT<CX>::mk(a.x + bb.y, -a.y + bb.x);
-        }
-      }
-    }
-    __syncwarp();
-    static_assert(NKXP - 1 == NX / 3, "the truncated band of the pruned pass is NX/3 + 1 ..");
-    wpasses_pz<NX, +1, PV, tp_ok(NX)>(buf, NPIN, SSTR, stw, lane);
-#pragma unroll
-    for (int q = 0; q < NPIN; q++)
-#pragma unroll
-      for (int i = 0; i < XPL; i++) {
-        const int x = lane + 32 * i;
-        const CX v = (x < NX) ? buf[q * SSTR + pad(x)] : CT<CX>::mk(0, 0);
-        dst[2 * q][i] = v.x;
-        if (2 * q + 1 < NF) dst[2 * q + 1][i] = v.y;
-      }
-    __syncwarp();
-  };
-
-  load_plane(j0 - 1, cur, dcur);
-  for (int j = j0 - 1; j <= j1; j++) {
-    load_plane(j + 1, nxt, dnxt);
-    const T dyf_j = dyf[j], dyf_p = dyf[j + 1], dy_p = dy[j + 1];
-    const T wgy = (T)1 / ((T)2 * dy_p);
-    // products: GYF j (U1U3, U1U1, U3U3, g, TH U1, TH U3) and GY j+1 (fl1, fl3,
-    // ubar1 u2, ubar3 u2, flth)
-    // FP32 form: row means of the products, P = L1 L2 with L = D + L'
-    double pdc[F32 ? NPROD : 1];
-    if constexpr (F32) {
-      double acc[NPROD];
-#pragma unroll
-      for (int p = 0; p < NPROD; p++) acc[p] = 0.0;
-      const double wgyd = 1.0 / (2. * (double)dy[j + 1]);
-      const double dfj = dyf[j], dfp = dyf[j + 1];
-      double L1d[NPROD], L2d[NPROD];
-      // (L1, L2) row means of each product, in the order of P[] below
-      L1d[0] = dcur[2]; L2d[0] = dcur[0];
-      L1d[1] = dcur[0]; L2d[1] = dcur[0];
-      L1d[2] = dcur[2]; L2d[2] = dcur[2];
-      L1d[3] = 0.5 * (dcur[1] + dnxt[1]); L2d[3] = L1d[3];
-      L1d[4] = dnxt[0] + dcur[0]; L2d[4] = dnxt[1];
-      L1d[5] = dnxt[2] + dcur[2]; L2d[5] = dnxt[1];
-      L1d[6] = (dfp * dnxt[0] + dfj * dcur[0]) * wgyd; L2d[6] = dnxt[1];
-      L1d[7] = (dfp * dnxt[2] + dfj * dcur[2]) * wgyd; L2d[7] = dnxt[1];
-#pragma unroll
-      for (int n = 0; n < NTH; n++) {
-        L1d[8 + 3 * n] = dcur[3 + n]; L2d[8 + 3 * n] = dcur[0];
-        L1d[9 + 3 * n] = dcur[3 + n]; L2d[9 + 3 * n] = dcur[2];
-        L1d[10 + 3 * n] = dnxt[3 + n] + dcur[3 + n]; L2d[10 + 3 * n] = dnxt[1];
-      }
-#pragma unroll
-      for (int i = 0; i < XPL; i++) {
-        const int x = lane + 32 * i;
-        if (x >= NX) continue;
-        const float u1 = cur[0][i], u2 = cur[1][i], u3 = cur[2][i];
-        const float u1p = nxt[0][i], u2p = nxt[1][i], u3p = nxt[2][i];
-        float L1f[NPROD], L2f[NPROD];
-        L1f[0] = u3; L2f[0] = u1;
-        L1f[1] = u1; L2f[1] = u1;
-        L1f[2] = u3; L2f[2] = u3;
-        L1f[3] = 0.5f * (u2 + u2p); L2f[3] = L1f[3];
-        L1f[4] = u1p + u1; L2f[4] = u2p;
-        L1f[5] = u3p + u3; L2f[5] = u2p;
-        L1f[6] = ((T)dyf_p * u1p + (T)dyf_j * u1) * wgy; L2f[6] = u2p;
-        L1f[7] = ((T)dyf_p * u3p + (T)dyf_j * u3) * wgy; L2f[7] = u2p;
-#pragma unroll
-        for (int n = 0; n < NTH; n++) {
-          const float t = cur[3 + n][i], tp = nxt[3 + n][i];
-          L1f[8 + 3 * n] = t; L2f[8 + 3 * n] = u1;
-          L1f[9 + 3 * n] = t; L2f[9 + 3 * n] = u3;
-          L1f[10 + 3 * n] = tp + t; L2f[10 + 3 * n] = u2p;
-        }
-        T P[2 * NPP];
-#pragma unroll
-        for (int p = 0; p < NPROD; p++) {
-          const float ff = L1f[p] * L2f[p];
-          // the row mean takes the exact product of the FP32 fluctuations (48
-          // significant bits fit FP64) and sums it in FP64: no FP32 rounding
-          // enters the mean, whatever the row length
-          acc[p] = fma((double)L1f[p], (double)L2f[p], acc[p]);
-          P[p] = (float)L1d[p] * L2f[p] + (float)L2d[p] * L1f[p] + ff;
-        }
-        if (2 * NPP > NPROD) P[2 * NPP - 1] = 0.0f;
-#pragma unroll
-        for (int q = 0; q < NPP; q++) buf[q * SSTR + pad(x)] = CT<CX>::mk(P[2 * q], P[2 * q + 1]);
-      }
-#pragma unroll
-      for (int p = 0; p < NPROD; p++) {
-        double v = acc[p];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        pdc[p] = L1d[p] * L2d[p] + v / (double)NX;
-      }
-    } else {
-#pragma unroll
-    for (int i = 0; i < XPL; i++) {
-      const int x = lane + 32 * i;
-      if (x >= NX) continue;
-      const T u1 = cur[0][i], u2 = cur[1][i], u3 = cur[2][i];
-      const T u1p = nxt[0][i], u2p = nxt[1][i], u3p = nxt[2][i];
-      T P[2 * NPP];
-      P[0] = u3 * u1;
-      P[1] = u1 * u1;
-      P[2] = u3 * u3;
-      { const T s = u2 + u2p; P[3] = (T)0.25 * (s * s); }
-      P[4] = (u1p + u1) * u2p;
-      P[5] = (u3p + u3) * u2p;
-      P[6] = ((dyf_p * u1p + dyf_j * u1) * wgy) * u2p;
-      P[7] = ((dyf_p * u3p + dyf_j * u3) * wgy) * u2p;
-#pragma unroll
-      for (int n = 0; n < NTH; n++) {
-        const T t = cur[3 + n][i], tp = nxt[3 + n][i];
-        P[8 + 3 * n] = t * u1;
-        P[9 + 3 * n] = t * u3;
-        P[10 + 3 * n] = (tp + t) * u2p;
-      }
-      if (2 * NPP > NPROD) P[2 * NPP - 1] = 0.0;
-#pragma unroll
-      for (int q = 0; q < NPP; q++) buf[q * SSTR + pad(x)] = CT<CX>::mk(P[2 * q], P[2 * q + 1]);
-    }
-    }
-    __syncwarp();
-    wpasses<NX, -1, 0, PV, tp_ok(NX)>(buf, NPP, SSTR, stw, lane);
-    const bool out = (j >= j0);
-    const T d2 = (T)2 * dyf_j, dyj = dy[j];
-    const T id2 = (T)1 / d2, idyj = (T)1 / dyj;  // per plane: multiply in the row loop
-#pragma unroll
-    for (int s = 0; s < KS; s++) {
-      const int k = lane + 32 * s;
-      if (k >= NKXP) continue;
-      auto X = [&](int p) -> CX {
-        if constexpr (F32) {
-          if (k == 0) return CT<CX>::mk((T)pdc[p], (T)0);
-        }
-        const int q = p >> 1;
-        const CX zk = buf[q * SSTR + pad(k)];
-        const CX zm = buf[q * SSTR + pad((NX - k) % NX)];
-        CX v;
-        if ((p & 1) == 0) v = CT<CX>::mk((T)0.5 * (zk.x + zm.x), (T)0.5 * (zk.y - zm.y));
-        else v = CT<CX>::mk((T)0.5 * (zk.y + zm.y), -(T)0.5 * (zk.x - zm.x));
-        if (pow2) return CT<CX>::mk(v.x * rnx, v.y * rnx);
-        return CT<CX>::mk(v.x / (T)NX, v.y / (T)NX);
-      };
-      const T KX = kxv[k];
-      auto mikx = [&](CX a) { return CT<CX>::mk(KX * a.y, -KX * a.x); };  // -i kx a
-      const CX x3 = X(3), x4 = X(4), x5 = X(5), x6 = X(6), x7 = X(7);
-      if (out) {
-        const long off = (long)j * NZ * NKXP + (long)z * NKXP + k;
-        const CX x0 = X(0), x1 = X(1), x2 = X(2);
-        // U1: A = U1U3, B = -ikx U1U1 - (fl1(j+1) - fl1(j)) / (2 DYF(j))
-        G[0 * Gfield + off] = x0;
-        CX t = mikx(x1);
-        G[1 * Gfield + off] = CT<CX>::mk(t.x - (x4.x - PV(0, s).x) * id2, t.y - (x4.y - PV(0, s).y) * id2);
-        // U2 (GY j): A = ubar3 u2(j), B = -ikx ubar1 u2(j) - (g(j) - g(j-1)) / DY(j)
-        G[2 * Gfield + off] = PV(3, s);
-        t = mikx(PV(2, s));
-        G[3 * Gfield + off] = CT<CX>::mk(t.x - (x3.x - PV(4, s).x) * idyj, t.y - (x3.y - PV(4, s).y) * idyj);
-        // U3: A = U3U3, B = -ikx U1U3 - (fl3(j+1) - fl3(j)) / (2 DYF(j))
-        G[4 * Gfield + off] = x2;
-        t = mikx(x0);
-        G[5 * Gfield + off] = CT<CX>::mk(t.x - (x5.x - PV(1, s).x) * id2, t.y - (x5.y - PV(1, s).y) * id2);
-#pragma unroll
-        for (int n = 0; n < NTH; n++) {
-          const CX a = X(8 + 3 * n), b = X(9 + 3 * n), c = X(10 + 3 * n);
-          G[(6 + 2 * n) * Gfield + off] = b;
-          t = mikx(a);
-          G[(7 + 2 * n) * Gfield + off] =
-              CT<CX>::mk(t.x - (c.x - PV(5 + n, s).x) * id2, t.y - (c.y - PV(5 + n, s).y) * id2);
-        }
-      }
-      PV(0, s) = x4;
-      PV(1, s) = x5;
-      PV(2, s) = x6;
-      PV(3, s) = x7;
-      PV(4, s) = x3;
-#pragma unroll
-      for (int n = 0; n < NTH; n++) PV(5 + n, s) = X(10 + 3 * n);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int f = 0; f < NF; f++) {
-#pragma unroll
-      for (int i = 0; i < XPL; i++) cur[f][i] = nxt[f][i];
-      dcur[f] = dnxt[f];
-    }
-  }
-#undef PV
-}
-
-template <int NX, int NTH, typename CX = double2>
-size_t xw_smem() {
-  constexpr int NF = 3 + NTH, NPIN = (NF + 1) / 2, NPP = (8 + 3 * NTH + 1) / 2;
-  constexpr int MAXP = NPIN > NPP ? NPIN : NPP;
-  return sizeof(CX) * (NX + XW_WARPS * MAXP * padded_len(NX) + XW_WARPS * (5 + NTH) * (NX / 3 + 1));
-}
-
-// the plan variant of the handle's tuning, for lengths that have one
-template <int NX, int NTH, typename CX>
-auto xrow_kernel(int v) {
-  if constexpr (plan_has_variant(NX))
-    if (v) return k_xrow_w<NX, NTH, CX, 1>;
-  return k_xrow_w<NX, NTH, CX, 0>;
 }
 
 // ------------------------------------------------------------- zfwd + rhs
@@ -1755,7 +1472,7 @@ __global__ void k_absmax(const double *__restrict__ a, long n, unsigned long lon
 }  // namespace
 
 // ================================================================ host side
-// Planes one CTA of a marching kernel takes (k_xrow_w, k_xmarch) when the
+// Planes one CTA of a marching kernel takes (k_xrows, k_xmarch) when the
 // tuning leaves it automatic (DG_TUNE_XROW_CHUNK = 0).  A CTA costs `per`
 // for each of its planes and `lead` for the planes it loads before the first
 // one; the chunk is the one whose waves of resident CTAs cost least in all.
@@ -2036,7 +1753,7 @@ int dg_chan_init(dg_handle *h) {
   return dg_cn_tables(h);
 }
 
-// The mixed form needs a compile-time x length (the warp x-row kernel, or
+// The mixed form needs a compile-time x length (k_xrows or k_xmarch, or
 // the FP32 two-launch stage) and a warp z-forward length.
 bool dg_mixed_ok(int nx, int nz, int n_th) {
   (void)n_th;
@@ -2059,35 +1776,11 @@ static int nl_chunk_mixed(dg_handle *h, const ChanConst &C, int rk_step, int a, 
   DG_TRY(zs);
   hdone = b + 1;
   const int nplan = b - a + 1;
-  bool done = false;
-#define XW_CASE(NXV, NTHV)                                                                      \
-  if (!done && h->NX == NXV && h->NTH == NTHV) {                                                \
-    auto kern = xrow_kernel<NXV, NTHV, float2>(h->fft_plan);                                    \
-    dg_big_smem((const void *)kern);                                                            \
-    int chunk = h->xrow_chunk > 0 ? (h->xrow_chunk < nplan ? h->xrow_chunk : nplan)            \
-                                  : dg_march_chunk(nplan, dg_cdiv(h->NZ, XW_WARPS),             \
-                                                   (const void *)kern, 32 * XW_WARPS,           \
-                                                   xw_smem<NXV, NTHV, float2>(), 1.0, 1.0);     \
-    dim3 grid(dg_cdiv(h->NZ, XW_WARPS), dg_cdiv(nplan, chunk));                                 \
-    dg_kt_begin(h, "k_xrow_w_f32", h->st);                                                      \
-    DG_CUDA(dg_launch(h->pdl, kern, grid, dim3(32 * XW_WARPS),                                  \
-                      xw_smem<NXV, NTHV, float2>(), h->st, C, Hf, Hfield, chunk, a, b,          \
-                      h->twx_f, h->dyf, h->dy, h->kx, Gf, Hfield));                             \
-    done = true;                                                                                \
-  }
-#define XW_ALL(NXV) XW_CASE(NXV, 0) XW_CASE(NXV, 1) XW_CASE(NXV, 2)
-  XW_ALL(16) XW_ALL(32) XW_ALL(48) XW_ALL(64) XW_ALL(96) XW_ALL(128) XW_ALL(256)
-#undef XW_ALL
-#undef XW_CASE
-  if (!done) {
-    dg_set_error("mixed precision: no FP32 x-row kernel for this NX / N_TH");
-    return DG_ERR_DIMS;
-  }
-  DG_LAUNCHED();
+  DG_TRY(dg_xrows(h, a, b));
   if (h->zf_nlo) return dg_cols_nl(h, a, b);
   dim3 zgrid(dg_cdiv(h->nkxp, zw_kxg(h->NZ)), nplan, h->nf);
   const size_t sm = zw_smem<float2>(h->NZ);
-  done = false;
+  bool done = false;
 #define ZW_CASE(N)                                                                              \
   if (!done && h->NZ == N) {                                                                    \
     auto kern = zfwd_kernel<N, float2>(h->fft_plan);                                            \
@@ -2109,7 +1802,7 @@ static int nl_chunk_mixed(dg_handle *h, const ChanConst &C, int rk_step, int a, 
   return DG_OK;
 }
 
-// Steps 1-3 in the mixed form for x lengths without an FP32 warp x-row
+// Steps 1-3 in the mixed form for x lengths that k_xrows does not take
 // kernel (or N_TH > 2): all planes at once through k_xc2r_f and k_xprod_f,
 // then the FP32 warp z-forward with its FP64 epilogue.
 static int nl_generic_mixed(dg_handle *h, const ChanConst &C, int rk_step,
@@ -2221,7 +1914,7 @@ int dg_chan_nonlinear(dg_handle *h, int time_step, int rk_step, bool *column_nex
   // the assembled right-hand side R and CF from it
   h->zf_nlo = les_solve ? 0 : 1;
   if (sgs) DG_TRY(dg_les_pre(h, rk_step));
-  if (h->mixed && !(xw_supported(h->NX) && h->NTH <= 2)) {
+  if (h->mixed && !dg_xrows_ok(h)) {
     DG_TRY(nl_generic_mixed(h, C, rk_step, in, cu, cf, rhs));
     a0 = h->NY + 1;  // every plane done: no chunk loop
   }
@@ -2239,30 +1932,9 @@ int dg_chan_nonlinear(dg_handle *h, int time_step, int rk_step, bool *column_nex
     hdone = b + 1;
     // 2. x-row nonlinear products for output planes a..b
     bool done = false;
-    if (xw_supported(h->NX) && h->NTH <= 2) {
-      const int nplan = b - a + 1;
-      // planes marched by one CTA (tunable DG_TUNE_XROW_CHUNK; 0 = the one-wave
-      // choice of xrow_auto_chunk)
-#define XW_CASE(NXV, NTHV)                                                                         \
-  if (h->NX == NXV && h->NTH == NTHV) {                                                          \
-    auto kern = xrow_kernel<NXV, NTHV, double2>(h->fft_plan);                                    \
-    dg_big_smem((const void *)kern);                                                             \
-    int chunk = h->xrow_chunk > 0 ? (h->xrow_chunk < nplan ? h->xrow_chunk : nplan)             \
-                                  : dg_march_chunk(nplan, dg_cdiv(h->NZ, XW_WARPS),             \
-                                                   (const void *)kern, 32 * XW_WARPS,           \
-                                                   xw_smem<NXV, NTHV>(), 1.0, 1.0);             \
-    dim3 grid(dg_cdiv(h->NZ, XW_WARPS), dg_cdiv(nplan, chunk));                                  \
-    dg_kt_begin(h, "k_xrow_w", h->st);                                                             \
-    DG_CUDA(dg_launch(h->pdl, kern, grid, dim3(32 * XW_WARPS),                                   \
-                      xw_smem<NXV, NTHV>(), h->st, C, h->H, Hfield, chunk, a, b, h->twx,        \
-                      h->dyf, h->dy, h->kx, h->G, Hfield));                                     \
-    done = true;                                                                                 \
-  }
-#define XW_ALL(NXV) XW_CASE(NXV, 0) XW_CASE(NXV, 1) XW_CASE(NXV, 2)
-      XW_ALL(16) XW_ALL(32) XW_ALL(48) XW_ALL(64) XW_ALL(96) XW_ALL(128) XW_ALL(256)
-#undef XW_ALL
-#undef XW_CASE
-      if (done) DG_LAUNCHED();
+    if (dg_xrows_ok(h)) {
+      DG_TRY(dg_xrows(h, a, b));
+      done = true;
     }
     if (!done) {
       // generic CTA kernel covers all planes 1..NY in one launch

@@ -1,5 +1,5 @@
-// The x-row stage of a channel substep for the row lengths that one warp
-// cannot hold (k_xrow_w takes 16..256): x c2r of every field, the products of
+// The x-row stage of a channel substep for the row lengths above those of
+// k_xrows (16..128): x c2r of every field, the products of
 // for/channel.f:409-571,665-720 and their x r2c, one CTA per z-row marching
 // up through a chunk of planes.
 //
@@ -32,7 +32,7 @@
 // differences are taken in physical space, so each pair maps onto the A/B
 // arrays of G.  With FP32 (mixed precision) every row is split into its mean
 // (FP64) and its fluctuation, and the means of the products are summed in
-// FP64 and put in the kx = 0 bin, as in k_xrow_w.
+// FP64 and put in the kx = 0 bin.
 #include <math.h>
 
 #include <type_traits>
@@ -500,6 +500,7 @@ int xm_dispatch(dg_handle *h, const CX *H, const CX *tw, CX *G, const char *name
     return xm_launch<T, R1, 2, CX>(h, H, tw, G, name);                 \
   }
   XM_CASE(192, 64, 3)
+  XM_CASE(256, 64, 4)
   XM_CASE(384, 128, 3)
   XM_CASE(512, 128, 4)
 #undef XM_CASE
@@ -509,7 +510,7 @@ int xm_dispatch(dg_handle *h, const CX *H, const CX *tw, CX *G, const char *name
 }  // namespace
 
 bool dg_xmarch_ok(const dg_handle *h) {
-  return (h->NX == 192 || h->NX == 384 || h->NX == 512) && h->NTH <= 2;
+  return (h->NX == 192 || h->NX == 256 || h->NX == 384 || h->NX == 512) && h->NTH <= 2;
 }
 
 int dg_xmarch(dg_handle *h) {

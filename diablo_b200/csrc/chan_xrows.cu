@@ -15,8 +15,13 @@
 //
 // A row and plane makes 2 trips through shared memory per inverse signal and 2 (and
 // the shuffles) per forward one, where passes between buffers (input, two
-// passes, output) made 6 each; that bandwidth bounded the stage.
-// @@MEASURED@@
+// passes, output) made 6 each; that bandwidth bounded the stage (60% of its
+// peak), which one warp per row with Stockham passes took 73 us for at
+// 128x129x128 and now takes 55 (events around eager launches): 29 -> 17 us at 128x65x32
+// with a scalar, 79 -> 31 at 96x65x96, 75 -> 45 at 64x129x128 with two; FP32
+// 59 -> 49 at 128x129x128.  Two CTAs per SM at up to 255 registers: a lane's points of two
+// planes and its RF values are registers (with 168 and spills 60 us; FP32
+// without scalars fits 168 and three CTAs, 49 us against 55).
 //
 // The pairs are those of k_xprod (chan_kernels.cu), as in k_xmarch; forward
 // signals go through in batches of NB = RF / RS, one item per lane.
@@ -57,7 +62,7 @@ __host__ __device__ constexpr int xr_buf(int RF, int RS, int nth) {
 }
 
 template <int RF, int RS, int NTH, typename CX>
-__global__ void __launch_bounds__(128, sizeof(CX) == 16 ? XR_B64 : XR_B32)
+__global__ void __launch_bounds__(128, sizeof(CX) == 8 && NTH == 0 ? 3 : 2)
     k_xrows(XrArgs A, const CX *__restrict__ H, const CX *__restrict__ tw, CX *__restrict__ G) {
   using TR = typename CT<CX>::T;
   constexpr bool F32 = sizeof(TR) == 4;
@@ -151,7 +156,7 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 16 ? XR_B64 : XR_B32)
     const double id2 = 1.0 / (2.0 * dyfj), idyj = 1.0 / A.dy[j];
     const TR cj = (TR)(dyfj * wgyd), cm = (TR)(dyfm * wgyd);
     auto old = [&](int f, int m) -> TR { return prv[(f * RS + m) * RF + t]; };
-    double acc[2 * NB];  // FP32 form: sums of the products of the fluctuations
+    double acc[2 * NB] = {};  // FP32 form: sums of the products of the fluctuations
     // FP32 form: (D1 + a)(D2 + b) without its mean part D1 D2; the sum of a b
     // goes to accumulator i in FP64
     auto pr = [&](double d1, TR a, double d2, TR b, int i, double sg) -> TR {
@@ -368,6 +373,9 @@ int xr_dispatch(dg_handle *h, int ja, int jb, const CX *H, const CX *tw, CX *G, 
 
 }  // namespace
 
+// (256 points would take 16 per lane and field, of two planes: in FP64 they do not fit the
+// registers, and in FP32 k_xmarch is faster, 70 us against 101 at 256x129x64 with a
+// scalar)
 bool dg_xrows_ok(const dg_handle *h) {
   const int n = h->NX;
   return h->NTH <= 2 && (n == 16 || n == 32 || n == 48 || n == 64 || n == 96 || n == 128);

@@ -549,3 +549,31 @@ def test_column_transforms_match_oracle(precision, nx, nz, n_th):
         ch.step(s)
     compare(ref, ch, fields(p), tol=TOL if precision == 0 else 1e-5)
     ch.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("nx,n_th,ny,nz,chunk", [
+    (16, 0, 9, 18, 0), (16, 2, 12, 16, 1), (32, 1, 17, 20, 3), (32, 2, 5, 48, 0), (48, 0, 9, 30, 9),
+    (48, 1, 21, 16, 4), (64, 0, 18, 36, 1), (64, 1, 4, 16, 0), (64, 2, 9, 54, 4), (96, 0, 13, 18, 5),
+    (96, 2, 8, 16, 0), (128, 0, 9, 30, 2), (128, 1, 16, 16, 16), (128, 2, 6, 20, 0),
+    (256, 0, 9, 16, 0), (256, 1, 10, 32, 4), (256, 2, 5, 16, 1)])
+def test_register_rows_match_oracle(nx, n_th, ny, nz, chunk, precision):
+    """The x-row stage with its points in registers (k_xrows, and k_xmarch at
+    256): every length and number of scalars, groups of rows that the last CTA
+    fills in part, whole and partial chunks of planes, FP64 and FP32, over 2
+    steps against the oracle (FP32: the mixed form's bar)."""
+    if precision and nz not in (16, 32, 48):
+        nz = 48 if nz > 32 else 32
+    p, gy = configs.channel_re180(nx=nx, ny=ny, nz=nz)
+    p = p.replace(n_th=n_th, precision=precision, variable_dt=0, delta_t=5e-4)
+    p.pr = [0.71, 1.3, 1, 1]
+    p.ri = [0.2, 0.0, 0, 0]
+    p.th_bc_ymin_c1 = [-1.0, 0.5, 0, 0]
+    p.th_bc_ymax_c1 = [1.0, -0.5, 0, 0]
+    ref, ch, _ = start_pair(p, gy, ics.channel_laminar, seed=41)
+    ch.tune_set(xrow_chunk=chunk)
+    for s in (1, 2):
+        ref.step(s)
+        ch.step(s)
+    compare(ref, ch, fields(p), tol=TOL if precision == 0 else 1e-5)
+    ch.close()
