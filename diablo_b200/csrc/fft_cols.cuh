@@ -83,6 +83,39 @@ template <> struct DFT<9> {
   }
 };
 
+// 32-point DFT as 4 x 8: n = 8 n1 + n2, k = k1 + 4 k2, twiddles exp(sign 2 pi i m / 32)
+template <> struct DFT<32> {
+  template <typename C> static __device__ __forceinline__ void run(C *v, int sign) {
+    using T = typename CT<C>::T;
+    // cos(2 pi m / 32), m = 0..24; sin(2 pi m / 32) = cos(2 pi (m - 8) / 32)
+    const T Q[9] = {(T)1.0, (T)0.98078528040323044913, (T)0.92387953251128675613,
+                    (T)0.83146961230254523708, (T)0.70710678118654752440, (T)0.55557023301960222474,
+                    (T)0.38268343236508977173, (T)0.19509032201612826785, (T)0.0};
+    C a[8][4];
+#pragma unroll
+    for (int n2 = 0; n2 < 8; n2++) {
+      C t[4] = {v[n2], v[8 + n2], v[16 + n2], v[24 + n2]};
+      DFT<4>::run(t, sign);
+#pragma unroll
+      for (int k1 = 0; k1 < 4; k1++) {
+        const int m = n2 * k1;  // 0..21
+        const T cs = m <= 8 ? Q[m] : m <= 16 ? -Q[16 - m] : -Q[m - 16];
+        const T sn = m <= 8 ? Q[8 - m] : m <= 16 ? Q[m - 8] : -Q[24 - m];
+        a[n2][k1] = m ? cmul(t[k1], CT<C>::mk(cs, sign * sn)) : t[k1];
+      }
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 4; k1++) {
+      C t[8];
+#pragma unroll
+      for (int n2 = 0; n2 < 8; n2++) t[n2] = a[n2][k1];
+      DFT<8>::run(t, sign);
+#pragma unroll
+      for (int k2 = 0; k2 < 8; k2++) v[k1 + 4 * k2] = t[k2];
+    }
+  }
+};
+
 // The split of a column length; rc = 1: two steps.
 struct ColPlan {
   int n, ra, rb, rc;

@@ -577,3 +577,28 @@ def test_register_rows_match_oracle(nx, n_th, ny, nz, chunk, precision):
         ch.step(s)
     compare(ref, ch, fields(p), tol=TOL if precision == 0 else 1e-5)
     ch.close()
+
+
+@pytest.mark.parametrize("nx,n_th,ny,nz,chunk", [
+    (20, 0, 9, 18, 0), (20, 2, 6, 30, 2), (24, 1, 17, 20, 3), (30, 0, 5, 16, 0), (30, 2, 9, 32, 9),
+    (36, 1, 12, 18, 1), (36, 2, 4, 16, 0), (40, 0, 18, 36, 4), (40, 2, 9, 20, 0), (54, 1, 13, 16, 5),
+    (60, 0, 8, 54, 0), (60, 2, 17, 18, 16), (72, 0, 6, 16, 2), (72, 2, 9, 20, 0), (80, 1, 10, 30, 3),
+    (90, 2, 8, 16, 0), (120, 0, 5, 18, 1), (120, 1, 9, 36, 0), (160, 0, 9, 20, 4), (160, 1, 6, 16, 0),
+    (160, 2, 17, 18, 6)])
+def test_register_rows_factor_5_and_9_match_oracle(nx, n_th, ny, nz, chunk):
+    """k_xrows at the lengths whose groups of lanes do not fill a warp, with
+    one item per lane and with idle lanes in its last step, over 2 steps
+    against the oracle."""
+    p, gy = configs.channel_re180(nx=nx, ny=ny, nz=nz)
+    p = p.replace(n_th=n_th, variable_dt=0, delta_t=5e-4)
+    p.pr = [0.71, 1.3, 1, 1]
+    p.ri = [0.2, 0.0, 0, 0]
+    p.th_bc_ymin_c1 = [-1.0, 0.5, 0, 0]
+    p.th_bc_ymax_c1 = [1.0, -0.5, 0, 0]
+    ref, ch, _ = start_pair(p, gy, ics.channel_laminar, seed=43)
+    ch.tune_set(xrow_chunk=chunk)
+    for s in (1, 2):
+        ref.step(s)
+        ch.step(s)
+    compare(ref, ch, fields(p))
+    ch.close()
