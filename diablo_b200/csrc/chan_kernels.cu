@@ -1802,8 +1802,8 @@ static int nl_chunk_mixed(dg_handle *h, const ChanConst &C, int rk_step, int a, 
   return DG_OK;
 }
 
-// Steps 1-3 in the mixed form for x lengths that k_xrows does not take
-// kernel (or N_TH > 2): all planes at once through k_xc2r_f and k_xprod_f,
+// Steps 1-3 in the mixed form for x lengths that neither k_xrows nor
+// k_xmarch takes (or N_TH > 2): all planes at once through k_xc2r_f and k_xprod_f,
 // then the FP32 warp z-forward with its FP64 epilogue.
 static int nl_generic_mixed(dg_handle *h, const ChanConst &C, int rk_step,
                             const double2 *const *in, FieldPtrs cu, FieldPtrs cf, FieldPtrs rhs) {

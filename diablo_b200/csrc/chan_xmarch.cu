@@ -1,5 +1,6 @@
-// The x-row stage of a channel substep for the row lengths above those of
-// k_xrows (16..128): x c2r of every field, the products of
+// The x-row stage of a channel substep for rows of 256 (with scalars), 384 and
+// 512 points, in FP32 of 192 and 256 too, which have too many points for the
+// registers of k_xrows (chan_xrows.cuh): x c2r of every field, the products of
 // for/channel.f:409-571,665-720 and their x r2c, one CTA per z-row marching
 // up through a chunk of planes.
 //
@@ -100,8 +101,8 @@ __device__ __forceinline__ void xm_first(CX *__restrict__ buf, int s0, int ns, i
 }
 
 // hides a value's origin from the compiler, so that what is computed from it
-// inside the plane loop is not kept in registers across it (FP64, T = 64: 192
-// -> 184 us at 192x97x192 with a scalar; the others measured slower with it)
+// inside the plane loop is not kept in registers across it (FP64, T = 64:
+// 4% faster per launch; the others measured slower with it)
 template <bool ON>
 __device__ __forceinline__ int xm_fresh(int v) {
   if constexpr (ON) asm volatile("" : "+r"(v));
@@ -493,24 +494,34 @@ int xm_launch(dg_handle *h, const CX *H, const CX *tw, CX *G, const char *name) 
 
 template <typename CX>
 int xm_dispatch(dg_handle *h, const CX *H, const CX *tw, CX *G, const char *name) {
-#define XM_CASE(N, T, R1)                                              \
-  if (h->NX == N) {                                                    \
-    if (h->NTH == 0) return xm_launch<T, R1, 0, CX>(h, H, tw, G, name); \
+#define XM_CASE(T, R1)                                               \
+  {                                                                  \
     if (h->NTH == 1) return xm_launch<T, R1, 1, CX>(h, H, tw, G, name); \
-    return xm_launch<T, R1, 2, CX>(h, H, tw, G, name);                 \
+    if (h->NTH == 2) return xm_launch<T, R1, 2, CX>(h, H, tw, G, name); \
   }
-  XM_CASE(192, 64, 3)
-  XM_CASE(256, 64, 4)
-  XM_CASE(384, 128, 3)
-  XM_CASE(512, 128, 4)
+#define XM_CASE0(T, R1) \
+  if (h->NTH == 0) return xm_launch<T, R1, 0, CX>(h, H, tw, G, name);
+  if (h->NX == 512) {
+    XM_CASE0(128, 4) XM_CASE(128, 4)
+  } else if (h->NX == 384) {
+    XM_CASE0(128, 3) XM_CASE(128, 3)
+  } else if (h->NX == 256) {
+    // without scalars in FP64: k_xrows
+    if constexpr (sizeof(CX) == 8) XM_CASE0(64, 4)
+    XM_CASE(64, 4)
+  } else if constexpr (sizeof(CX) == 8) {
+    XM_CASE0(64, 3) XM_CASE(64, 3)
+  }
 #undef XM_CASE
+#undef XM_CASE0
   return DG_ERR_ARG;
 }
 
 }  // namespace
 
 bool dg_xmarch_ok(const dg_handle *h) {
-  return (h->NX == 192 || h->NX == 256 || h->NX == 384 || h->NX == 512) && h->NTH <= 2;
+  return ((h->NX == 192 && h->mixed) || h->NX == 256 || h->NX == 384 || h->NX == 512) &&
+         h->NTH <= 2 && !dg_xrows_ok(h);
 }
 
 int dg_xmarch(dg_handle *h) {

@@ -17,13 +17,10 @@ int xr_dispatch(dg_handle *h, int ja, int jb, const CX *H, const CX *tw, CX *G, 
 
 }  // namespace
 
-// (256 points would take 16 per lane and field, of two planes: in FP64 they do not fit the
-// registers, and in FP32 k_xmarch is faster, 70 us against 101 at 256x129x64 with a
-// scalar)
 bool dg_xrows_ok(const dg_handle *h) {
   const int n = h->NX;
   const bool both = n == 16 || n == 32 || n == 48 || n == 64 || n == 96 || n == 128;
-  return h->NTH <= 2 && (both || (!h->mixed && dg_xrows5_ok(n)));
+  return h->NTH <= 2 && (both || (!h->mixed && dg_xrows64_ok(n, h->NTH)));
 }
 
 // output planes ja..jb (H holds ja-1..jb+1)
@@ -31,6 +28,6 @@ int dg_xrows(dg_handle *h, int ja, int jb) {
   if (h->mixed)
     return xr_dispatch(h, ja, jb, reinterpret_cast<const float2 *>(h->H), (const float2 *)h->twx_f,
                        reinterpret_cast<float2 *>(h->G), "k_xrows_f32");
-  if (dg_xrows5_ok(h->NX)) return dg_xrows5(h, ja, jb);
+  if (dg_xrows64_ok(h->NX, h->NTH)) return dg_xrows64(h, ja, jb);
   return xr_dispatch(h, ja, jb, (const double2 *)h->H, (const double2 *)h->twx, h->G, "k_xrows");
 }

@@ -1,9 +1,9 @@
-// k_xrows (chan_xrows.cuh) for lengths with a factor 5 or 9, FP64: the longer ones.
+// k_xrows (chan_xrows.cuh) for 72 to 160 points, FP64.
 #include "chan_xrows.cuh"
 
-int dg_xrows5_long(dg_handle *h, int ja, int jb);
+int dg_xrows64_l(dg_handle *h, int ja, int jb);
 
-int dg_xrows5_long(dg_handle *h, int ja, int jb) {
+int dg_xrows64_l(dg_handle *h, int ja, int jb) {
   const double2 *H = h->H, *tw = h->twx;
   switch (h->NX) {
     case 72: return xr_th<9, 8, double2>(h, ja, jb, H, tw, h->G, "k_xrows");

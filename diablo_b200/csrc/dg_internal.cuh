@@ -255,8 +255,8 @@ bool dg_xmarch_ok(const dg_handle *h);  // the x-row stage runs as k_xmarch
 int dg_xmarch(dg_handle *h);
 bool dg_xrows_ok(const dg_handle *h);   // or as k_xrows
 int dg_xrows(dg_handle *h, int ja, int jb);
-bool dg_xrows5_ok(int n);               // lengths with a factor 5 or 9 (FP64)
-int dg_xrows5(dg_handle *h, int ja, int jb);
+bool dg_xrows64_ok(int n, int nth);               // the lengths of FP64 only
+int dg_xrows64(dg_handle *h, int ja, int jb);
 int dg_rem_div_dev(dg_handle *h, int update_cp, int rk_step, bool from_rhs);
 int dg_courant_dev(dg_handle *h, const double2 *const *u, bool side = false);
 int dg_stats_dev(dg_handle *h, dg_stats *s);

@@ -53,6 +53,7 @@ template <> struct DFT<6> : DFTpf<2, 3, 3, 4> {};
 template <> struct DFT<10> : DFTpf<2, 5, 5, 6> {};
 template <> struct DFT<12> : DFTpf<4, 3, 9, 4> {};
 template <> struct DFT<15> : DFTpf<3, 5, 10, 6> {};
+template <> struct DFT<20> : DFTpf<4, 5, 5, 16> {};
 
 // 9-point DFT as 3 x 3: n = 3 n1 + n2, k = k1 + 3 k2, twiddles exp(sign 2 pi i m / 9)
 template <> struct DFT<9> {
@@ -82,6 +83,10 @@ template <> struct DFT<9> {
     }
   }
 };
+
+template <> struct DFT<18> : DFTpf<2, 9, 9, 10> {};
+template <> struct DFT<24> : DFTpf<3, 8, 16, 9> {};
+template <> struct DFT<30> : DFTpf<5, 6, 6, 25> {};
 
 // 32-point DFT as 4 x 8: n = 8 n1 + n2, k = k1 + 4 k2, twiddles exp(sign 2 pi i m / 32)
 template <> struct DFT<32> {

@@ -584,7 +584,10 @@ def test_register_rows_match_oracle(nx, n_th, ny, nz, chunk, precision):
     (36, 1, 12, 18, 1), (36, 2, 4, 16, 0), (40, 0, 18, 36, 4), (40, 2, 9, 20, 0), (54, 1, 13, 16, 5),
     (60, 0, 8, 54, 0), (60, 2, 17, 18, 16), (72, 0, 6, 16, 2), (72, 2, 9, 20, 0), (80, 1, 10, 30, 3),
     (90, 2, 8, 16, 0), (120, 0, 5, 18, 1), (120, 1, 9, 36, 0), (160, 0, 9, 20, 4), (160, 1, 6, 16, 0),
-    (160, 2, 17, 18, 6)])
+    (160, 2, 17, 18, 6), (50, 1, 9, 16, 0), (100, 2, 6, 18, 2), (108, 0, 8, 16, 3), (144, 1, 5, 30, 0),
+    (150, 2, 9, 16, 4), (162, 1, 6, 18, 0), (180, 0, 9, 16, 1), (192, 1, 8, 20, 3),
+    (216, 2, 5, 16, 0), (240, 1, 9, 18, 5), (256, 0, 12, 16, 4), (270, 0, 6, 16, 0), (288, 1, 5, 18, 2),
+    (320, 2, 8, 16, 0)])
 def test_register_rows_factor_5_and_9_match_oracle(nx, n_th, ny, nz, chunk):
     """k_xrows at the lengths whose groups of lanes do not fill a warp, with
     one item per lane and with idle lanes in its last step, over 2 steps
