@@ -5,7 +5,7 @@
 // modes, packed like kz).  One substep:
 //   yinv   spectral -> Hy [y][kz][kx]       (c2c along y per (kz, kx) column)
 //   zinv   Hy -> H [y][z][kx]               (c2c along z per kx column)
-//   k_prod_per_w  per physical (y, z) row: x c2r of U1..U3 (and TH), the 6
+//   k_per_rows  (per_rows.cu) per physical (y, z) row: x c2r of U1..U3 (and TH), the 6
 //          (+3 per scalar) products u_i u_j, x r2c -> Hp [p][y][z][kx] / NX
 //   zfwd   Hp -> Qz [p][y][kz][kx] / NZ
 //   yfwd   Qz -> Fy [p][ky][kz][kx] / NY
@@ -48,115 +48,6 @@ PerConst make_pc(const dg_handle *h) {
     c.ri[n] = h->p.ri[n]; c.pr[n] = h->p.pr[n]; c.bg[n] = h->p.background_grad[n];
   }
   return c;
-}
-
-// ----------------------------------------------------------- products (warp)
-// One warp per physical (y, z) row: c2r of the fields, products, r2c.
-template <int NX, int NTH, typename CX = double2>
-__global__ void __launch_bounds__(128) k_prod_per_w(PerConst C, const CX *__restrict__ H,
-                                                    long Hfield, const CX *__restrict__ tw,
-                                                    CX *__restrict__ Hp, long Pfield) {
-  constexpr int NF = 3 + NTH;
-  constexpr int NPIN = (NF + 1) / 2;
-  constexpr int NPROD = 6 + 3 * NTH;
-  constexpr int NPP = (NPROD + 1) / 2;
-  constexpr int MAXP = NPIN > NPP ? NPIN : NPP;
-  constexpr int XPL = (NX + 31) / 32;
-  constexpr int NKXP = NX / 3 + 1;
-  constexpr int KS = (NKXP + 31) / 32;
-  constexpr int SSTR = padded_len(NX);
-  extern __shared__ double2 sm_raw[];
-  using T = typename CT<CX>::T;
-  CX *sm = reinterpret_cast<CX *>(sm_raw);
-  CX *stw = sm;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  CX *buf = stw + NX + warp * MAXP * SSTR;
-  for (int i = threadIdx.x; i < NX; i += blockDim.x) stw[i] = tw[i];
-  __syncthreads();
-  const long row = (long)blockIdx.x * 4 + warp;  // row = y * NZ + z
-  if (row >= (long)C.NY * C.NZ) return;
-  const CX *src = H + row * NKXP;
-  // c2r of field pairs
-#pragma unroll
-  for (int q = 0; q < NPIN; q++) {
-    const int fa = 2 * q, fb = 2 * q + 1;
-#pragma unroll
-    for (int i = 0; i < (NX + 31) / 32; i++) {
-      const int k = lane + 32 * i;
-      if (k < NX) {
-        const int kk = (k <= NX / 2) ? k : NX - k;
-        CX v = CT<CX>::mk(0, 0);
-        if (kk < NKXP && kk < NX / 2) {
-          CX a = src[fa * Hfield + kk];
-          CX b = (fb < NF) ? src[fb * Hfield + kk] : CT<CX>::mk(0, 0);
-          if (kk == 0) { a.y = 0.0; b.y = 0.0; }
-          v = (k == kk) ? CT<CX>::mk(a.x - b.y, a.y + b.x) : CT<CX>::mk(a.x + b.y, -a.y + b.x);
-        }
-        buf[q * SSTR + pad(k)] = v;
-      }
-    }
-  }
-  __syncwarp();
-  wpasses<NX, +1, 0>(buf, NPIN, SSTR, stw, lane);
-  T u[NF][XPL];
-#pragma unroll
-  for (int q = 0; q < NPIN; q++)
-#pragma unroll
-    for (int i = 0; i < XPL; i++) {
-      const int x = lane + 32 * i;
-      const CX v = (x < NX) ? buf[q * SSTR + pad(x)] : CT<CX>::mk(0, 0);
-      u[2 * q][i] = v.x;
-      if (2 * q + 1 < NF) u[2 * q + 1][i] = v.y;
-    }
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < XPL; i++) {
-    const int x = lane + 32 * i;
-    if (x >= NX) continue;
-    const T u1 = u[0][i], u2 = u[1][i], u3 = u[2][i];
-    T P[2 * NPP];
-    P[0] = u1 * u1;
-    P[1] = u1 * u2;
-    P[2] = u1 * u3;
-    P[3] = u2 * u2;
-    P[4] = u2 * u3;
-    P[5] = u3 * u3;
-#pragma unroll
-    for (int n = 0; n < NTH; n++) {
-      const T t = u[3 + n][i];
-      P[6 + 3 * n] = u1 * t;
-      P[7 + 3 * n] = u2 * t;
-      P[8 + 3 * n] = u3 * t;
-    }
-    if (2 * NPP > NPROD) P[2 * NPP - 1] = 0.0;
-#pragma unroll
-    for (int q = 0; q < NPP; q++) buf[q * SSTR + pad(x)] = CT<CX>::mk(P[2 * q], P[2 * q + 1]);
-  }
-  __syncwarp();
-  wpasses<NX, -1, 0>(buf, NPP, SSTR, stw, lane);
-  CX *dst = Hp + row * NKXP;
-#pragma unroll
-  for (int s = 0; s < KS; s++) {
-    const int k = lane + 32 * s;
-    if (k >= NKXP) continue;
-#pragma unroll
-    for (int p = 0; p < NPROD; p++) {
-      const int q = p >> 1;
-      const CX zk = buf[q * SSTR + pad(k)];
-      const CX zm = buf[q * SSTR + pad((NX - k) % NX)];
-      CX v;
-      if ((p & 1) == 0) v = CT<CX>::mk((T)0.5 * (zk.x + zm.x), (T)0.5 * (zk.y - zm.y));
-      else v = CT<CX>::mk((T)0.5 * (zk.y + zm.y), -(T)0.5 * (zk.x - zm.x));
-      dst[p * Pfield + k] = CT<CX>::mk(v.x / (T)NX, v.y / (T)NX);
-    }
-  }
-}
-
-template <int NX, int NTH, typename CX = double2>
-size_t prod_smem() {
-  constexpr int NF = 3 + NTH, NPIN = (NF + 1) / 2, NPP = (6 + 3 * NTH + 1) / 2;
-  constexpr int MAXP = NPIN > NPP ? NPIN : NPP;
-  return sizeof(CX) * (NX + 4 * MAXP * padded_len(NX));
 }
 
 // generic products from physical fields (any NX): phys [f][y][z][x] -> prod [p][y][z][x]
@@ -462,12 +353,6 @@ int per_to_fourier(dg_handle *h, const double *src, int nf, double2 *const *fiel
   return per_to_fourier(h, src, nf, phys_field(h), (long)h->NZ * h->NX, h->NX, fields);
 }
 
-// whether k_prod_per_w has a specialisation for this NX and N_TH
-bool prod_warp_ok(const dg_handle *h) {
-  const int n = h->NX;
-  return h->NTH <= 2 && (n == 16 || n == 32 || n == 48 || n == 64 || n == 96 || n == 128 || n == 256);
-}
-
 }  // namespace
 
 int dg_per_init(dg_handle *h) {
@@ -486,8 +371,8 @@ int dg_per_init(dg_handle *h) {
   DG_TRY(al(&h->P, (size_t)nmax * h_field(h)));        // Hp
   DG_TRY(al(&h->Q, (size_t)np * fy_field(h)));         // Fy
   // physical scratch: 6 fields for POISSON_P_PER; the generic product path
-  // (lengths or scalar counts without a warp specialisation) needs nf + np
-  const int nphys = prod_warp_ok(h) ? 6 : (h->nf + np > 6 ? h->nf + np : 6);
+  // (lengths or scalar counts that k_per_rows does not take) needs nf + np
+  const int nphys = dg_per_rows_ok(h->NX, h->NTH) ? 6 : (h->nf + np > 6 ? h->nf + np : 6);
   h->work_bytes = sizeof(double) * (size_t)phys_field(h) * nphys;
   if (h->work_bytes < sizeof(double) * 8 * (size_t)h->nkyt)
     h->work_bytes = sizeof(double) * 8 * (size_t)h->nkyt;
@@ -527,25 +412,11 @@ static int per_nonlinear_mixed(dg_handle *h, const PerConst &C) {
   for (int f = 0; f < nf; f++) hy[f] = Hyf + f * hy_field(h);
   DG_TRY(dg_cinv_ff(h, hy, nf, 0, h->NY - 1, h->ss, h->nkxp, h->NZ, h->NKZ, h->plz, h->twz_f, Hf,
                     h_field(h)));
-  bool done = false;
-  const long rows = (long)h->NY * h->NZ;
-#define PW_CASE(NXV, NTHV)                                                                      \
-  if (!done && h->NX == NXV && h->NTH == NTHV) {                                                \
-    dg_big_smem((const void *)k_prod_per_w<NXV, NTHV, float2>);                                 \
-    dg_kt_begin(h, "k_prod_per_w_f32", h->st);                                                  \
-    k_prod_per_w<NXV, NTHV, float2><<<dg_cdiv(rows, 4), 128, prod_smem<NXV, NTHV, float2>(),    \
-                                      h->st>>>(C, Hf, h_field(h), h->twx_f, Pf, h_field(h));    \
-    done = true;                                                                                \
-  }
-#define PW_ALL(NXV) PW_CASE(NXV, 0) PW_CASE(NXV, 1) PW_CASE(NXV, 2)
-  PW_ALL(16) PW_ALL(32) PW_ALL(48) PW_ALL(64) PW_ALL(96) PW_ALL(128) PW_ALL(256)
-#undef PW_ALL
-#undef PW_CASE
-  if (!done) {
+  if (!dg_per_rows_ok(h->NX, h->NTH)) {
     dg_set_error("mixed precision: no FP32 product kernel for this NX / N_TH");
     return DG_ERR_DIMS;
   }
-  DG_LAUNCHED();
+  DG_TRY(dg_per_rows(h));
   float2 *qz[6 + 3 * DG_MAX_TH], *fy[6 + 3 * DG_MAX_TH];
   for (int p = 0; p < np; p++) {
     qz[p] = Hyf + p * hy_field(h);
@@ -602,22 +473,8 @@ extern "C" int diablo_rk_per_1(dg_handle *h, int rk_step) {
   DG_TRY(dg_cinv_g(h, hy, nf, 0, h->NY - 1, h->ss, h->nkxp, h->NZ, h->NKZ, h->plz, h->twz, h->H,
                    h_field(h)));
   // x rows: products
-  bool done = false;
-  const long rows = (long)h->NY * h->NZ;
-#define PW_CASE(NXV, NTHV)                                                                     \
-  if (!done && h->NX == NXV && h->NTH == NTHV) {                                               \
-    dg_big_smem((const void *)k_prod_per_w<NXV, NTHV>);                                        \
-    dg_kt_begin(h, "k_prod_per_w", h->st);                                                       \
-    k_prod_per_w<NXV, NTHV><<<dg_cdiv(rows, 4), 128, prod_smem<NXV, NTHV>(), h->st>>>(          \
-        C, h->H, h_field(h), h->twx, h->P, h_field(h));                                       \
-    done = true;                                                                               \
-  }
-#define PW_ALL(NXV) PW_CASE(NXV, 0) PW_CASE(NXV, 1) PW_CASE(NXV, 2)
-  PW_ALL(16) PW_ALL(32) PW_ALL(48) PW_ALL(64) PW_ALL(96) PW_ALL(128) PW_ALL(256)
-#undef PW_ALL
-#undef PW_CASE
-  if (done) {
-    DG_LAUNCHED();
+  if (dg_per_rows_ok(h->NX, h->NTH)) {
+    DG_TRY(dg_per_rows(h));
   } else {
     // generic: physical fields, pointwise products, r2c of each product
     double *phys = (double *)h->work;

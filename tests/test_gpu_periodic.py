@@ -212,3 +212,21 @@ def test_graph_steps_match_substep_calls():
         assert np.array_equal(a.get_field(nm), b.get_field(nm)), nm
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("nx,nth", [
+    (16, 0), (16, 2), (20, 1), (24, 0), (30, 2), (32, 0), (36, 1), (40, 0), (48, 2), (50, 1), (54, 0),
+    (60, 2), (64, 1), (72, 0), (80, 1), (90, 2), (96, 0), (100, 1), (108, 2), (120, 0), (128, 2),
+    (144, 1), (150, 0), (160, 2), (162, 1), (180, 0), (192, 2), (200, 1), (216, 0), (240, 2), (256, 0),
+    (256, 1), (256, 2), (270, 1), (288, 2), (320, 0)])
+def test_product_rows_match_oracle(nx, nth):
+    """Every row length of the product kernel, with a last block that is not full (100 rows)."""
+    p = box((nx, 10, 10), n_th=nth)
+    p.ri = [0.3, -0.2, 0, 0]
+    p.pr = [0.7, 1.5, 1, 1]
+    ref, g = seeded_pair(p, seed=nx + nth, scalars=[0.5] * nth)
+    ref.step(1)
+    g.step(1)
+    for nm in fields(p) + ["CF1", "CF2", "CF3"]:
+        assert rel(g.get_field(nm), ref.get(nm)) <= TOL, nm
+    g.close()
