@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(PL_THR, 2) k_plane_c2r(CFieldPtrs fields, int 
       }
     }
     __syncwarp();
-    wpasses_pz<NXT, +1, 0, false>(xw, np, SX, twx, lane);
+    wpasses_pz<NXT, +1>(xw, np, SX, twx, lane);
     for (int q = 0; q < np; q++) {
       const int za = 2 * (p0 + q), zb = za + 1;
 #pragma unroll
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(PL_THR, 2) k_plane_r2c(const double *__restric
       }
     __syncwarp();
     if (p0 + PSTEP < NZT / 2) fetch(p0 + PSTEP);
-    wpasses_any<NXT, -1, 0, 0, false>(xw, np, SX, twx, lane);
+    wpasses_any<NXT, -1, 0>(xw, np, SX, twx, lane);
     for (int q = 0; q < np; q++) {
       const int za = 2 * (p0 + q), zb = za + 1;
       for (int k = lane; k < NKXP; k += 32) {
