@@ -73,10 +73,11 @@ def kernel_bytes_per_launch(p, name):
     Mh, Mi = L * NZ * nkxp, NY * NZ * nkxp  # half-physical values, all / interior planes
     c = 16
     table = {
-        "k_zinv": c * nf * (M + Mh),
-        "k_xrow_w": c * (nf * Mh + 2 * nf * Mi),
+        "k_cols_inv": c * nf * (M + Mh),
+        "k_xrows": c * (nf * Mh + 2 * nf * Mi),
+        "k_xmarch": c * (nf * Mh + 2 * nf * Mi),
         # z forward of the 2 Nf product arrays; writes NL of every field
-        "k_zfwd_w": c * (2 * nf * Mi + nf * Si),
+        "k_cols_nl": c * (2 * nf * Mi + nf * Si),
         # column stage, all fields: read CU, NL, CF_old and CP (once); write
         # CF and the post-CN field
         "k_col_cn": c * (2 * nf * M + nf * Si * (1 + 2 / 3 + 1) + M),

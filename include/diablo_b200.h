@@ -222,7 +222,7 @@ int dg_timing_read(dg_handle *h, int i, char *name, int name_len, int64_t *launc
 /* No counterpart in the reference.  Launch shapes of the channel substep:
  * modes per CTA of the REM_DIV y-column kernel (4, 8, 16) and of the substep's
  * column kernel (one field's right-hand side and CN solve; 2, 4, 8, 16),
- * y-planes per CTA of the x-row product kernel (0 = automatic), planes per
+ * y-planes per CTA of the x-row product kernels (0 = automatic), planes per
  * y-chunk of a substep (0 = all).  Results do not depend on them
  * (DG_TUNE_FFT_PLAN below: at round-off level only).  dg_autotune times
  * candidates on the handle's own state (steps_per_trial eager RK3 steps each), keeps the
@@ -235,10 +235,11 @@ enum { DG_TUNE_COL_MT = 0, DG_TUNE_XROW_CHUNK = 1, DG_TUNE_YCHUNK = 2, DG_TUNE_C
  * where the x and z lengths allow (16, 32, 48, 64, 96 or 128); 0 stages them
  * through a half-physical array in two launches.  Same transforms, same
  * results; the setting is not tuned. */
-/* DG_TUNE_FFT_PLAN: radix order of the x and z transform plans of the
- * substep (0: largest radix first, 128 = 16 x 8; 1: the reverse, 8 x 16).
- * The same transform either way; the autotuner times both per grid shape.
- * Unlike the other tunables it changes the order of the transforms'
+/* DG_TUNE_FFT_PLAN: radix order of the transforms that run as passes in
+ * shared memory (0: largest radix first, 128 = 16 x 8; 1: the reverse, 8 x 16):
+ * the z forward with LES and COURANT's x transform.  The others split their
+ * length one way.  The same transform either way; the autotuner times both per
+ * grid shape.  Unlike the other tunables it changes the order of the transforms'
  * arithmetic, so results differ between the two at round-off level (both
  * are held to the same parity tolerance). */
 /* DG_TUNE_WAIT_TEST (test only): value > 0 makes the next Crank-Nicolson
