@@ -1,4 +1,6 @@
-// Shared-memory mixed-radix Stockham FFT used by all transform kernels.
+// Shared-memory mixed-radix Stockham FFT of the kernels that run a transform as
+// passes (k_xmarch, the whole planes of LES, COURANT, lengths without a split in
+// fft_cols.cuh or chan_xrows.cuh), and the butterflies of all.
 //
 // A batch of `nsig` complex signals of length N lives in shared memory, one
 // signal per `sig_stride` double2, element i of a signal stored at pad(i) =
@@ -14,9 +16,9 @@
 // inverse direction conjugates it.  Unnormalised in both directions, which
 // is FFTW's convention (forward sign -1).
 //
-// Two front ends: run<N>() with the transform length and radix plan fixed at
+// Two front ends: fft_cta<N>() with the transform length and radix plan fixed at
 // compile time (all index arithmetic folds), and run() with a runtime plan
-// for lengths without a specialisation.
+// for lengths without a specialisation (N = 0).
 #pragma once
 
 #include <cuda_runtime.h>
