@@ -12,8 +12,9 @@
 // of one lane: what bound the passes was shared memory and its latency.
 //
 // Measured per launch, from one warp per row with those passes: FP64 256^3 368 ->
-// 228 us (6 arrays of 86 x 256^2 bins written, 3 read: 6.3 TB/s of H and P), with a scalar
-// 256x64x128 81 -> 50, 128^3 53 -> 31, 32^3 8.6 -> 7.4; FP32 128^3 33 -> 23,
+// 225 us (6 arrays of 86 x 256^2 bins written, 3 read: 812 MB at 3.6 TB/s; with 255
+// registers 8 warps share an SM, and the latency of loads and FP64 bounds it), with a
+// scalar 256x64x128 81 -> 50, 128^3 53 -> 31, 32^3 8.6 -> 7.4; FP32 128^3 33 -> 23,
 // 96x64x96 with a scalar 25 -> 15.  The lengths with a factor 5 or 9, FP64 only, took
 // a c2r launch per field, the products through physical arrays and an r2c launch
 // per product: 192x64x64 with a scalar 204 -> 25 us, 100x64x64 156 -> 17.
