@@ -1771,7 +1771,7 @@ static int nl_chunk_mixed(dg_handle *h, const ChanConst &C, int rk_step, int a, 
   const long Hfield = (long)h->nplanes * h->NZ * h->nkxp;
   h->pdl_zinv = h->pdl;  // follows the previous substep's REM_DIV kernel
   const int zs = dg_cinv_gf(h, in, h->nf, hdone + 1, b + 1, h->ss, h->nkxp, h->NZ, h->NKZ, h->plz,
-                            h->twz_f, Hf, Hfield);
+                            h->twz_f, Hf, Hfield, dg_peak_out(h));
   h->pdl_zinv = 0;
   DG_TRY(zs);
   hdone = b + 1;
@@ -1813,7 +1813,7 @@ static int nl_generic_mixed(dg_handle *h, const ChanConst &C, int rk_step,
   const int NX = h->NX, NY = h->NY, NZ = h->NZ;
   h->pdl_zinv = h->pdl;
   const int zs = dg_cinv_gf(h, in, h->nf, 0, NY + 1, h->ss, h->nkxp, NZ, h->NKZ, h->plz, h->twz_f,
-                            Hf, Hfield);
+                            Hf, Hfield, dg_peak_out(h));
   h->pdl_zinv = 0;
   DG_TRY(zs);
   bool done = false;
@@ -1926,7 +1926,8 @@ int dg_chan_nonlinear(dg_handle *h, int time_step, int rk_step, bool *column_nex
     }
     // 1. z inverse of the planes this chunk's x-rows need (a-1 .. b+1)
     h->pdl_zinv = h->pdl;
-    const int zs = dg_zinv(h, in, h->nf, hdone + 1, b + 1, h->H, false);
+    const PeakOut peak = dg_xrows_ok(h) || dg_xmarch_ok(h) ? dg_peak_out(h) : PeakOut();
+    const int zs = dg_zinv(h, in, h->nf, hdone + 1, b + 1, h->H, false, peak);
     h->pdl_zinv = 0;
     DG_TRY(zs);
     hdone = b + 1;
@@ -1939,7 +1940,7 @@ int dg_chan_nonlinear(dg_handle *h, int time_step, int rk_step, bool *column_nex
     if (!done) {
       // generic CTA kernel covers all planes 1..NY in one launch
       if (a == 1) {
-        DG_TRY(dg_zinv(h, in, h->nf, hdone + 1, h->NY + 1, h->H, false));
+        DG_TRY(dg_zinv(h, in, h->nf, hdone + 1, h->NY + 1, h->H, false, peak));
         hdone = h->NY + 1;
         if (dg_xmarch_ok(h)) {
           DG_TRY(dg_xmarch(h));

@@ -63,10 +63,8 @@ __host__ __device__ constexpr int xm_signals(int nth) {
   return xm_pairs(nth) > (4 + nth) / 2 ? xm_pairs(nth) : (4 + nth) / 2;
 }
 
-// fields of the inverse's signal s: (U1, TH1), (U2, U3), (TH2, TH3).  The
-// rounding of a packed transform is relative to the larger of its two rows,
-// and U1 (the stream) is larger than U2 and U3: packed with U2 it cost the
-// FP32 form 1.17 times its error.
+// fields of the inverse's signal s: (U1, TH1), TH1 scaled to U1's magnitude
+// (dg_pair_shift); (U2, U3), (TH2, -)
 __host__ __device__ constexpr int xm_fa(int s) { return s < 2 ? s : 2 * s; }
 __host__ __device__ constexpr int xm_fb(int s) { return s == 0 ? 3 : s == 1 ? 2 : 2 * s + 1; }
 
@@ -75,6 +73,8 @@ struct XmArgs {
   long Hfield, Gfield;
   int chunk, jbase, jtop;
   const double *dyf, *dy, *kx;
+  const unsigned *peak;  // of H's planes
+  int planes, plen;
 };
 
 // first pass of the inverse sub-transforms s0 .. s0+ns-1: radix R, inputs
@@ -172,6 +172,14 @@ __device__ __forceinline__ double xm_lane_sums(double (&v)[16], int lane) {
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
+// out of line: inlined, it moved the register allocation of the plane loop (512 points
+// with a scalar in FP64: 588 bytes of spills and 2.82 ms per launch, 232 and 2.12 so)
+template <typename T, int NTH>
+__device__ __noinline__ void xm_plane_shifts(int *sh, const unsigned *peak, int planes, int len,
+                                             int pl0, int n) {
+  dg_plane_shifts<T, NTH>(sh, peak, planes, len, pl0, n);
+}
+
 template <int T, int R1, int NTH, typename CX>
 __global__ void __launch_bounds__(T, (T == 128 ? 1 : 2) * (sizeof(CX) == 16 ? 3 : 4)) k_xmarch(
     XmArgs A, const CX *__restrict__ H, const CX *__restrict__ tw, CX *__restrict__ G) {
@@ -189,6 +197,7 @@ __global__ void __launch_bounds__(T, (T == 128 ? 1 : 2) * (sizeof(CX) == 16 ? 3 
   CX *stw = reinterpret_cast<CX *>(sm_raw);       // twiddles of length T
   CX *buf = stw + T;                              // [signal][q][SSTR]
   TR *prv = reinterpret_cast<TR *>(buf + xm_signals(NTH) * R1 * SSTR);  // [field][r][T], plane j-1
+  int *shf = reinterpret_cast<int *>(prv + NF * NX);  // shifts of the chunk's planes
   __shared__ double red[F32 ? NW : 1][16];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int z = blockIdx.x, NZ = A.NZ;
@@ -213,11 +222,22 @@ __global__ void __launch_bounds__(T, (T == 128 ? 1 : 2) * (sizeof(CX) == 16 ? 3 
   TR cur[NF][R1], nxt[NF][R1];
   double dcur[NF], dnxt[NF], dprv[NF];  // row means (FP32 form)
 
-  auto load_plane = [&](int pl, TR (&dst)[NF][R1], double (&dcv)[NF]) {
+  if constexpr (NTH > 0)
+    xm_plane_shifts<TR, NTH>(shf, A.peak, A.planes, A.plen, j0 - 1, j1 - j0 + 3);
+  int shc = 0, shn = 0;  // two scalars: TH2's shift to TH1 in their common pair, planes j and j+1
+  auto load_plane = [&](int pl, TR (&dst)[NF][R1], double (&dcv)[NF], int &sh) {
     const CX *row = Hz + (long)pl * plane;
+    const int sw = NTH > 0 ? shf[pl - j0 + 1] : 0, d = (short)sw;  // TH1 goes times 2^d
     if constexpr (F32) {
 #pragma unroll
       for (int f = 0; f < NF; f++) dcv[f] = (double)__ldg(row + f * A.Hfield).x;
+    }
+    if constexpr (NTH == 2) {
+      if constexpr (F32)  // the products hold the row means, the peaks do not
+        sh = dg_pair_shift<TR>(max((sw >> 24) & 255, dg_mag_exp<TR>(dg_mag((TR)dcv[3]))),
+                               max((sw >> 16) & 255, dg_mag_exp<TR>(dg_mag((TR)dcv[4]))), 0);
+      else
+        sh = sw >> 16;
     }
     constexpr int NS = NPIN * R1, PER = (NS + NW - 1) / NW;
     const int ln = xm_fresh<T == 64 && sizeof(CX) == 16>(lane), s0 = xm_fresh<T == 64 && sizeof(CX) == 16>(warp) * PER, ns = min(PER, NS - s0);
@@ -227,6 +247,7 @@ __global__ void __launch_bounds__(T, (T == 128 ? 1 : 2) * (sizeof(CX) == 16 ? 3 
         const int q = sub % R1, s = sub / R1, fb = xm_fb(s);
         const CX *ra = row + xm_fa(s) * A.Hfield, *rb = row + fb * A.Hfield;
         const bool two = fb < NF;
+        const TR sc = dg_pow2<TR>(NTH > 0 && s == 0 ? d : 0);
 #pragma unroll
         for (int r = 0; r < R0; r++) {
           if (R1 * r * NB0 > KLO && R1 * (r * NB0 + NB0) - 1 < KHI) {
@@ -241,7 +262,8 @@ __global__ void __launch_bounds__(T, (T == 128 ? 1 : 2) * (sizeof(CX) == 16 ? 3 
             if (two) c = __ldg(rb + kk);
             if (kk == 0) a.y = c.y = 0;
           }
-          v[r] = (k == kk) ? CT<CX>::mk(a.x - c.y, a.y + c.x) : CT<CX>::mk(a.x + c.y, c.x - a.y);
+          v[r] = (k == kk) ? CT<CX>::mk(a.x - sc * c.y, a.y + sc * c.x)
+                           : CT<CX>::mk(a.x + sc * c.y, sc * c.x - a.y);
         }
       });
       xm_passes<T, +1, 1, 0, 0>(buf + s0 * SSTR, ns, SSTR, stw, xm_fresh<T == 64 && sizeof(CX) == 16>(ln));
@@ -259,18 +281,19 @@ __global__ void __launch_bounds__(T, (T == 128 ? 1 : 2) * (sizeof(CX) == 16 ? 3 
 #pragma unroll
       for (int r = 0; r < R1; r++) {
         dst[xm_fa(s)][r] = v[r].x;
-        if (xm_fb(s) < NF) dst[xm_fb(s)][r] = v[r].y;
+        if (xm_fb(s) < NF)
+          dst[xm_fb(s)][r] = s == 0 ? v[r].y * dg_pow2<TR>(-d) : v[r].y;
       }
     }
     __syncthreads();
   };
 
-  load_plane(j0 - 1, cur, dprv);
+  load_plane(j0 - 1, cur, dprv, shc);
 #pragma unroll
   for (int f = 0; f < NF; f++)
 #pragma unroll
     for (int r = 0; r < R1; r++) prv[(f * R1 + r) * T + t] = cur[f][r];
-  load_plane(j0, cur, dcur);
+  load_plane(j0, cur, dcur, shc);
   for (int j = j0; j <= j1; j++) {
     // the row that the next step reads comes from HBM: into L2 meanwhile
     if (j < j1) {
@@ -281,7 +304,7 @@ __global__ void __launch_bounds__(T, (T == 128 ? 1 : 2) * (sizeof(CX) == 16 ? 3 
         asm volatile("prefetch.global.L2 [%0];" ::"l"(row + off));
       }
     }
-    load_plane(j + 1, nxt, dnxt);
+    load_plane(j + 1, nxt, dnxt, shn);
     const double dyfj = A.dyf[j], dyfm = A.dyf[j - 1], wgyd = 1.0 / (2.0 * A.dy[j]);
     const TR cj = (TR)(dyfj * wgyd), cm = (TR)(dyfm * wgyd);
     double acc[16];  // FP32 form: sums of the products of the fluctuations
@@ -340,8 +363,9 @@ __global__ void __launch_bounds__(T, (T == 128 ? 1 : 2) * (sizeof(CX) == 16 ? 3 
         return CT<CX>::mk(prod(f, 0, r, m), rise(f, r, m + 1));
       }
       const int n = 2 * (s - 4 - NTH), m = 8 + 2 * NTH + n;
-      return CT<CX>::mk(prod(3 + n, 2, r, m),
-                        n + 1 < NTH ? prod(4 + n < NF ? 4 + n : 3, 2, r, m + 1) : (TR)0);
+      return CT<CX>::mk(
+          prod(3 + n, 2, r, m),
+          n + 1 < NTH ? dg_pow2<TR>(shc) * prod(4 + n < NF ? 4 + n : 3, 2, r, m + 1) : (TR)0);
     };
 #pragma unroll
     for (int s = 0; s < NPP; s++) {
@@ -389,6 +413,10 @@ __global__ void __launch_bounds__(T, (T == 128 ? 1 : 2) * (sizeof(CX) == 16 ? 3 
         // B = -i/2 (Z_k - conj Z_{N-k})
         double2 a = make_double2(hx * ((double)zk.x + zm.x), hx * ((double)zk.y - zm.y));
         double2 b = make_double2(hx * ((double)zk.y + zm.y), -hx * ((double)zk.x - zm.x));
+        if (NTH == 2 && s == 4 + NTH) {
+          b.x *= dg_pow2<double>(-shc);
+          b.y *= dg_pow2<double>(-shc);
+        }
         if constexpr (F32) {
           if (k == 0) {
             // the row means of the pair's products
@@ -453,6 +481,7 @@ __global__ void __launch_bounds__(T, (T == 128 ? 1 : 2) * (sizeof(CX) == 16 ? 3 
         }
       }
     }
+    shc = shn;
     if constexpr (F32) {
 #pragma unroll
       for (int f = 0; f < NF; f++) {
@@ -468,21 +497,22 @@ __global__ void __launch_bounds__(T, (T == 128 ? 1 : 2) * (sizeof(CX) == 16 ? 3 
 // memory at NX = 512 with a scalar), four in FP32 (128 registers: 485 -> 390 us
 // at 512x65x384 with a scalar)
 template <int T, int R1, int NTH, typename CX>
-size_t xm_smem() {
+size_t xm_smem(int ny) {
   return sizeof(CX) * (T + (size_t)xm_signals(NTH) * R1 * xm_sstr(T, R1, (int)sizeof(CX))) +
-         sizeof(typename CT<CX>::T) * (3 + NTH) * (size_t)T * R1;
+         sizeof(typename CT<CX>::T) * (3 + NTH) * (size_t)T * R1 + (NTH > 0 ? sizeof(int) * (ny + 2) : 0);
 }
 
 template <int T, int R1, int NTH, typename CX>
 int xm_launch(dg_handle *h, const CX *H, const CX *tw, CX *G, const char *name) {
   auto kern = k_xmarch<T, R1, NTH, CX>;
-  const size_t sm = xm_smem<T, R1, NTH, CX>();
+  const size_t sm = xm_smem<T, R1, NTH, CX>(h->NY);
   dg_big_smem((const void *)kern);
   XmArgs A;
   A.NY = h->NY; A.NZ = h->NZ;
   A.Hfield = A.Gfield = (long)h->nplanes * h->NZ * h->nkxp;
   A.jbase = 1; A.jtop = h->NY;
   A.dyf = h->dyf; A.dy = h->dy; A.kx = h->kx;
+  A.peak = h->peak; A.planes = h->NY + 2; A.plen = h->peak_len;
   A.chunk = h->xrow_chunk > 0 ? (h->xrow_chunk < h->NY ? h->xrow_chunk : h->NY)
                               : dg_march_chunk(h->NY, h->NZ, (const void *)kern, T, sm, 1.0, 0.7);
   dg_kt_begin(h, name, h->st);

@@ -24,7 +24,10 @@
 // without scalars fits 168 and three CTAs, 49 us against 55).
 //
 // The pairs are those of k_xprod (chan_kernels.cu), as in k_xmarch; forward
-// signals go through in batches of NB = RF / RS, one item per lane.
+// signals go through in batches of NB = RF / RS, one item per lane.  Members that
+// have different units are brought to one magnitude by a power of two before a transform
+// and back after it (dg_pair_shift): a scalar packed with U1, the second scalar
+// packed with the first.
 #pragma once
 
 #include <math.h>
@@ -41,6 +44,8 @@ struct XrArgs {
   long Hfield, Gfield;
   int chunk, jbase, jtop;
   const double *dyf, *dy, *kx;
+  const unsigned *peak;  // of H's planes
+  int planes, plen;
 };
 
 __host__ __device__ constexpr int xr_pairs(int nth) { return 4 + nth + (nth + 1) / 2; }
@@ -81,6 +86,8 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 8 && NTH == 0 ? 3 : 2)
   constexpr int rows = (128 / 32) * RPW;
   CX *buf = reinterpret_cast<CX *>(sm_raw) + row * BUF;
   TR *prv = reinterpret_cast<TR *>(reinterpret_cast<CX *>(sm_raw) + rows * BUF) + row * (NF * NX);
+  int *shf = reinterpret_cast<int *>(
+      reinterpret_cast<TR *>(reinterpret_cast<CX *>(sm_raw) + rows * BUF) + rows * (NF * NX));
   const int NZ = A.NZ, zr = blockIdx.x * rows + row;
   const bool live = on && zr < NZ;  // a warp's rows step together
   const int z = zr < NZ ? zr : NZ - 1;
@@ -96,11 +103,22 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 8 && NTH == 0 ? 3 : 2)
   TR cur[NF][RS], nxt[NF][RS];
   double dcur[NF], dnxt[NF], dprv[NF];  // row means (FP32 form)
 
-  auto load_plane = [&](int pl, TR (&dst)[NF][RS], double (&dcv)[NF]) {
+  if constexpr (NTH > 0)
+    dg_plane_shifts<TR, NTH>(shf, A.peak, A.planes, A.plen, j0 - 1, j1 - j0 + 3);
+  int shc = 0, shn = 0;  // two scalars: TH2's shift to TH1 in their common pair, planes j and j+1
+  auto load_plane = [&](int pl, TR (&dst)[NF][RS], double (&dcv)[NF], int &sh) {
     const CX *src = Hz + (long)pl * plane;
+    const int sw = NTH > 0 ? shf[pl - j0 + 1] : 0, d = (short)sw;  // TH1 goes times 2^d
     if constexpr (F32) {
 #pragma unroll
       for (int f = 0; f < NF; f++) dcv[f] = (double)__ldg(src + f * A.Hfield).x;
+    }
+    if constexpr (NTH == 2) {
+      if constexpr (F32)  // the products hold the row means, the peaks do not
+        sh = dg_pair_shift<TR>(max((sw >> 24) & 255, dg_mag_exp<TR>(dg_mag((TR)dcv[3]))),
+                               max((sw >> 16) & 255, dg_mag_exp<TR>(dg_mag((TR)dcv[4]))), 0);
+      else
+        sh = sw >> 16;
     }
 #pragma unroll
     for (int i0 = 0; i0 < NPIN * RS; i0 += RF) {
@@ -108,6 +126,7 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 8 && NTH == 0 ? 3 : 2)
       if (on && i < NPIN * RS) {
         const CX *ra = src + xr_fa(s) * A.Hfield, *rb = src + xr_fb(s) * A.Hfield;
         const bool two = xr_fb(s) < NF;
+        const TR sc = dg_pow2<TR>(NTH > 0 && s == 0 ? d : 0);
         CX v[RF];
 #pragma unroll
         for (int r = 0; r < RF; r++) {
@@ -121,7 +140,8 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 8 && NTH == 0 ? 3 : 2)
             if (two) c = __ldg(rb + kk);
             if (kk == 0) a.y = c.y = 0;
           }
-          v[r] = (k == kk) ? CT<CX>::mk(a.x - c.y, a.y + c.x) : CT<CX>::mk(a.x + c.y, c.x - a.y);
+          v[r] = (k == kk) ? CT<CX>::mk(a.x - sc * c.y, a.y + sc * c.x)
+                           : CT<CX>::mk(a.x + sc * c.y, sc * c.x - a.y);
         }
         dft<RF>(v, +1);
         CX *o = buf + s * SI + b;
@@ -142,22 +162,23 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 8 && NTH == 0 ? 3 : 2)
 #pragma unroll
       for (int m = 0; m < RS; m++) {
         dst[xr_fa(s)][m] = v[m].x;
-        if (xr_fb(s) < NF) dst[xr_fb(s)][m] = v[m].y;
+        if (xr_fb(s) < NF)
+          dst[xr_fb(s)][m] = s == 0 ? v[m].y * dg_pow2<TR>(-d) : v[m].y;
       }
     }
     __syncwarp();
   };
 
-  load_plane(j0 - 1, cur, dprv);
+  load_plane(j0 - 1, cur, dprv, shc);
 #pragma unroll
   for (int f = 0; f < NF; f++)
 #pragma unroll
     for (int m = 0; m < RS; m++)
       if (on) prv[(f * RS + m) * RF + t] = cur[f][m];
-  load_plane(j0, cur, dcur);
+  load_plane(j0, cur, dcur, shc);
 #pragma unroll 1
   for (int j = j0; j <= j1; j++) {
-    load_plane(j + 1, nxt, dnxt);
+    load_plane(j + 1, nxt, dnxt, shn);
     const double dyfj = A.dyf[j], dyfm = A.dyf[j - 1], wgyd = 1.0 / (2.0 * A.dy[j]);
     const double id2 = 1.0 / (2.0 * dyfj), idyj = 1.0 / A.dy[j];
     const TR cj = (TR)(dyfj * wgyd), cm = (TR)(dyfm * wgyd);
@@ -211,7 +232,8 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 8 && NTH == 0 ? 3 : 2)
         return CT<CX>::mk(prod(f, 0, m, i), rise(f, m, i + 1));
       }
       const int n = 2 * (s - 4 - NTH), f = 3 + n < NF ? 3 + n : 0, g = 4 + n < NF ? 4 + n : 0;
-      return CT<CX>::mk(prod(f, 2, m, i), n + 1 < NTH ? prod(g, 2, m, i + 1) : (TR)0);
+      return CT<CX>::mk(prod(f, 2, m, i),
+                        n + 1 < NTH ? dg_pow2<TR>(shc) * prod(g, 2, m, i + 1) : (TR)0);
     };
     // mean parts of the pair's products
     auto means = [&](int s, double &da, double &db) {
@@ -299,6 +321,12 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 8 && NTH == 0 ? 3 : 2)
         // B = -i/2 (Z_k - conj Z_{N-k})
         double2 a = make_double2(hx * ((double)zk.x + zm.x), hx * ((double)zk.y - zm.y));
         double2 b = make_double2(hx * ((double)zk.y + zm.y), -hx * ((double)zk.x - zm.x));
+        if constexpr (NTH == 2) {
+          if (s0 + sl == 4 + NTH) {
+            b.x *= dg_pow2<double>(-shc);
+            b.y *= dg_pow2<double>(-shc);
+          }
+        }
         if constexpr (F32) {
           if (m == 0 && k == 0) {
             double da = 0.0, db = 0.0;
@@ -321,6 +349,7 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 8 && NTH == 0 ? 3 : 2)
       __syncwarp();
     }
     // plane j becomes j-1, j+1 becomes j
+    shc = shn;
 #pragma unroll
     for (int f = 0; f < NF; f++) {
 #pragma unroll
@@ -345,9 +374,11 @@ int xr_launch(dg_handle *h, int ja, int jb, const CX *H, const CX *tw, CX *G, co
   A.Hfield = A.Gfield = (long)h->nplanes * h->NZ * h->nkxp;
   A.jbase = ja; A.jtop = jb;
   A.dyf = h->dyf; A.dy = h->dy; A.kx = h->kx;
+  A.peak = h->peak; A.planes = h->NY + 2; A.plen = h->peak_len;
   constexpr int rows = 4 * (32 / RF);
   const size_t sm = sizeof(CX) * rows * (size_t)xr_buf(RF, RS, NTH) +
-                    sizeof(typename CT<CX>::T) * rows * (3 + NTH) * (size_t)(RF * RS);
+                    sizeof(typename CT<CX>::T) * rows * (3 + NTH) * (size_t)(RF * RS) +
+                    (NTH > 0 ? sizeof(int) * (h->NY + 2) : 0);
   const int nplan = jb - ja + 1, zb = dg_cdiv(h->NZ, rows);
   A.chunk = h->xrow_chunk > 0 ? (h->xrow_chunk < nplan ? h->xrow_chunk : nplan)
                               : dg_march_chunk(nplan, zb, (const void *)kern, 128, sm, 1.0, 0.7);

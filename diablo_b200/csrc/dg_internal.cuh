@@ -125,6 +125,8 @@ struct dg_handle {
   size_t work_bytes;
   unsigned long long *dmin_bits;// CFL min as ordered bits
   int *dflag;                   // non-finite flag
+  unsigned *peak;               // largest coefficients of H's planes (PeakOut) [nf][planes][peak_len]
+  int peak_len;
 
   // periodic extras
   double2 *Hy;                  // y-inverse output [nf][NY][nkzt][nkxp]
@@ -196,16 +198,28 @@ void dg_kt_end();
 void dg_kt_free(dg_handle *h);
 
 // common kernel-launch helpers (defined in fft_kernels.cu)
+// Where an inverse column transform leaves the largest component of what it writes
+// per field and plane, one value per warp: the bits of its absolute value (double:
+// the high word).  The row kernels take the power of two from it that brings two
+// packed fields to one magnitude (dg_pair_shift).  null: not wanted.
+struct PeakOut {
+  unsigned *p = nullptr;  // [nf][planes][dg_peak_len]
+  int planes = 0;
+  bool skip0 = false;     // without column 0 (row means, which the FP32 rows leave out)
+};
+int dg_peak_len(int n, int rowlen);  // values per field and plane
+PeakOut dg_peak_out(const dg_handle *h);  // h->peak: the substep's z inverse to rows of points
+int dg_cols_group(int n);            // columns per CTA of dg_cols_inv (0: no split)
 int dg_cinv_g(dg_handle *h, const double2 *const *fields, int nf, int jmin, int jmax,
               long in_plane, int rowlen, int N, int NK, const FftPlan &pl, const double2 *tw,
-              double2 *H, long out_field);
+              double2 *H, long out_field, PeakOut peak = {});
 // FP32 working precision (mixed path): FP64 spectral input, FP32 output
 int dg_cinv_gf(dg_handle *h, const double2 *const *fields, int nf, int jmin, int jmax,
                long in_plane, int rowlen, int N, int NK, const FftPlan &pl, const float2 *tw,
-               float2 *H, long out_field);
+               float2 *H, long out_field, PeakOut peak = {});
 int dg_cinv_ff(dg_handle *h, const float2 *const *fields, int nf, int jmin, int jmax,
                long in_plane, int rowlen, int N, int NK, const FftPlan &pl, const float2 *tw,
-               float2 *H, long out_field);
+               float2 *H, long out_field, PeakOut peak = {});
 int dg_cfwd_ff(dg_handle *h, const float2 *H, long in_field, int nf, int jmin, int jmax,
                int rowlen, int nkt, int N, int NK, const FftPlan &pl, const float2 *tw,
                float2 *const *fields, long out_plane);
@@ -215,11 +229,14 @@ int dg_cfwd_g(dg_handle *h, const double2 *H, long in_field, int nf, int jmin, i
 // the same transforms with one exchange through shared memory (fft_cols.cu);
 // 1 where the length has no such split
 int dg_cols_inv(dg_handle *h, const double2 *const *f, int nf, int jmin, int jmax, long in_plane,
-                int rowlen, int n, int nk, const double2 *tw, double2 *H, long out_field);
+                int rowlen, int n, int nk, const double2 *tw, double2 *H, long out_field,
+                PeakOut peak = {});
 int dg_cols_inv(dg_handle *h, const double2 *const *f, int nf, int jmin, int jmax, long in_plane,
-                int rowlen, int n, int nk, const float2 *tw, float2 *H, long out_field);
+                int rowlen, int n, int nk, const float2 *tw, float2 *H, long out_field,
+                PeakOut peak = {});
 int dg_cols_inv(dg_handle *h, const float2 *const *f, int nf, int jmin, int jmax, long in_plane,
-                int rowlen, int n, int nk, const float2 *tw, float2 *H, long out_field);
+                int rowlen, int n, int nk, const float2 *tw, float2 *H, long out_field,
+                PeakOut peak = {});
 int dg_cols_fwd(dg_handle *h, const double2 *H, long in_field, int nf, int jmin, int jmax,
                 int rowlen, int n, int nk, const double2 *tw, double2 *const *f, long out_plane);
 int dg_cols_fwd(dg_handle *h, const float2 *H, long in_field, int nf, int jmin, int jmax,
@@ -229,7 +246,7 @@ int dg_cols_nl(dg_handle *h, int jmin, int jmax);
 // plane_form: the passes of the whole-plane kernels (dg_plane_c2r, dg_plane_r2c), where
 // they exist for the lengths, so that the staged pair gives the same bits
 int dg_zinv(dg_handle *h, const double2 *const *fields, int nf, int jmin, int jmax,
-            double2 *H, bool plane_form);
+            double2 *H, bool plane_form, PeakOut peak = {});
 int dg_xc2r_planes(dg_handle *h, const double2 *H, int nf, int jmin, int jmax, double *phys,
                    long phys_plane_stride, long phys_row_stride, long field_stride);
 int dg_xc2r_cfl(dg_handle *h, const double2 *H, int jmin, int jmax, unsigned long long *out);
@@ -310,6 +327,66 @@ static inline int dg_cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 // trigger at kernel entry measured slower: the waiting CTAs held SM slots).
 // dg_pdl_wait() is a no-op for a plain launch.
 __device__ __forceinline__ void dg_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// ------------------------------------------------------------ packed rows
+// Two real rows in one complex transform: its rounding is relative to the larger
+// of the two, so that a scalar packed with U1 as it comes has the accuracy of U1's
+// unit, not of its own.  Its row goes times 2^d first and its points times 2^-d after the
+// transform, which is exact.  Errors after 4 steps in FP32 against FP64, 512x65x64, the scalar
+// 1/50 of U1's size: 1.0e-6 packed as it comes, 2.7e-9 with the shift (2.3e-9 with
+// transforms of two rows of one field); 128x65x64 4.9e-7 and 3.4e-9.
+__device__ __forceinline__ unsigned dg_mag(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned dg_mag(double x) { return __double2hiint(x) & 0x7fffffffu; }
+// biased exponent of a PeakOut value
+template <typename T> __device__ __forceinline__ int dg_mag_exp(unsigned m) {
+  return (int)(m >> (sizeof(T) == 4 ? 23 : 20));
+}
+// biased exponent of the largest of a field's len values of one plane
+template <typename T>
+__device__ __forceinline__ int dg_peak_exp(const unsigned *__restrict__ p, int len) {
+  unsigned m = 0;
+#pragma unroll 4
+  for (int i = 0; i < len; i += 4) {  // len is a multiple of 4, and so are the planes' offsets
+    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p + i));
+    m = max(max(m, max(v.x, v.y)), max(v.z, v.w));
+  }
+  return dg_mag_exp<T>(m);
+}
+// d for members with the biased exponents ea and eb: the second `below` binary orders
+// under the first.  One for a scalar with U1, whose error all fields see (U2's is
+// 1.01 times what it is beside a small scalar, 1.05 with none).  No shift where a member
+// is all zeros (or denormal) or not finite; the limit keeps 2^d and what it scales in range.
+template <typename T> __device__ __forceinline__ int dg_pair_shift(int ea, int eb, int below) {
+  constexpr int TOP = sizeof(T) == 4 ? 255 : 2047, LIM = sizeof(T) == 4 ? 60 : 500;
+  if (ea == 0 || eb == 0 || ea == TOP || eb == TOP) return 0;
+  return max(-LIM, min(LIM, ea - eb - below));
+}
+template <typename T> __device__ __forceinline__ T dg_pow2(int d) {
+  if constexpr (sizeof(T) == 4) return __int_as_float((127 + d) << 23);
+  else return __hiloint2double((1023 + d) << 20, 0);
+}
+
+// For a marching kernel, by its CTA before the first plane: the shifts of planes pl0 .. pl0+n-1
+// to sh[], from the peaks of [field][planes][len].  Low half: TH1 to U1.  With
+// two scalars the high half: TH2 to TH1 (double) or their two exponents (float, whose
+// rows add their means).  Once per plane in shared memory: with a reduction by each warp
+// at each of its planes k_xrows took 90 us at 160x98x60 with two scalars, 79 so (76 without the shifts).
+template <typename T, int NTH>
+__device__ __forceinline__ void dg_plane_shifts(int *sh, const unsigned *__restrict__ peak,
+                                                int planes, int len, int pl0, int n) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const unsigned *p = peak + (long)(pl0 + i) * len;
+    const long fs = (long)planes * len;
+    const int e0 = dg_peak_exp<T>(p, len), e1 = dg_peak_exp<T>(p + 3 * fs, len);
+    int hi = 0;
+    if constexpr (NTH == 2) {
+      const int e2 = dg_peak_exp<T>(p + 4 * fs, len);
+      hi = sizeof(T) == 4 ? e1 << 8 | e2 : dg_pair_shift<T>(e1, e2, 0);
+    }
+    sh[i] = (hi << 16) | (dg_pair_shift<T>(e0, e1, 1) & 0xffff);
+  }
+  __syncthreads();
+}
+
 // ------------------------------------------------------------ bulk copies
 // Bulk copies (cp.async.bulk, no multicast) into shared memory,
 // completed on an mbarrier.  Waits are bounded: a copy that does not land

@@ -40,15 +40,24 @@ struct LoadBins {
   }
 };
 
-template <typename CX>
+// PK: *pk becomes the largest component's magnitude of the columns but cskip
+template <typename CX, bool PK>
 struct StoreBins {
   CX *out;
   int rowlen, ncol;
+  unsigned *pk;
+  int cskip;
   template <int R>
   __device__ __forceinline__ void put(CX *v, int o, int step, int c, CX *, int) const {
     if (c >= ncol) return;
 #pragma unroll
     for (int m = 0; m < R; m++) out[(long)(o + m * step) * rowlen + c] = v[m];
+    if constexpr (PK) {
+      unsigned t = 0;
+#pragma unroll
+      for (int m = 0; m < R; m++) t = max(t, max(dg_mag(v[m].x), dg_mag(v[m].y)));
+      if (c != cskip) *pk = max(*pk, t);
+    }
   }
 };
 
@@ -73,10 +82,10 @@ struct StoreModes {
   }
 };
 
-template <int NT, typename CI, typename CX>
+template <int NT, bool PK, typename CI, typename CX>
 __global__ void __launch_bounds__(COLS_THR, 4)
     k_cols_inv(PtrArray<const CI> fields, int jmin, long in_plane, int rowlen, int nk, ColPlan pl,
-               int lk, const CX *__restrict__ tw, CX *__restrict__ H, long out_field) {
+               int lk, const CX *__restrict__ tw, CX *__restrict__ H, long out_field, PeakOut peak) {
   extern __shared__ double2 sm_raw[];
   CX *sm = reinterpret_cast<CX *>(sm_raw);
   const int n = NT ? NT : pl.n, kxg = 1 << (NT ? cols_log_kxg(NT) : lk);
@@ -85,8 +94,16 @@ __global__ void __launch_bounds__(COLS_THR, 4)
   dg_pdl_wait();
   cols_front<NT, +1>(sm, pl, lk, tw,
                      LoadModes<CI, CX>{fields(f) + (long)j * in_plane + c0, n, nk, rowlen, ncol});
+  unsigned pk = 0;
   cols_back<NT, +1>(sm, pl, lk,
-                    StoreBins<CX>{H + f * out_field + (long)j * n * rowlen + c0, rowlen, ncol});
+                    StoreBins<CX, PK>{H + f * out_field + (long)j * n * rowlen + c0, rowlen, ncol,
+                                      &pk, peak.skip0 && c0 == 0 ? 0 : -1});
+  if constexpr (PK) {
+    pk = __reduce_max_sync(0xffffffffu, pk);
+    if ((threadIdx.x & 31) == 0)
+      peak.p[(((long)f * peak.planes + j) * gridDim.x + blockIdx.x) * (COLS_THR / 32) +
+             (threadIdx.x >> 5)] = pk;
+  }
 }
 
 template <int NT, typename CX, typename CO>
@@ -199,7 +216,8 @@ bool cols_shape(int n, ColPlan *pl, int *lk, size_t *sm) {
 
 template <typename CI, typename CX>
 int inv_t(dg_handle *h, const CI *const *fields, int nf, int jmin, int jmax, long in_plane,
-          int rowlen, int n, int nk, const CX *tw, CX *H, long out_field, const char *name) {
+          int rowlen, int n, int nk, const CX *tw, CX *H, long out_field, PeakOut peak,
+          const char *name) {
   ColPlan pl;
   int lk;
   size_t sm;
@@ -210,11 +228,11 @@ int inv_t(dg_handle *h, const CI *const *fields, int nf, int jmin, int jmax, lon
   const dim3 grid(dg_cdiv(rowlen, 1 << lk), jmax - jmin + 1, nf);
 #define KERNEL_BODY(NN)                                                                        \
   {                                                                                            \
-    auto kern = k_cols_inv<NN, CI, CX>;                                                        \
+    auto kern = peak.p ? k_cols_inv<NN, true, CI, CX> : k_cols_inv<NN, false, CI, CX>;         \
     dg_big_smem((const void *)kern);                                                           \
     dg_kt_begin(h, name, h->st);                                                               \
     DG_CUDA(dg_launch(h->pdl_zinv, kern, grid, dim3(COLS_THR), sm, h->st, fp, jmin, in_plane,  \
-                      rowlen, nk, pl, lk, tw, H, out_field));                                  \
+                      rowlen, nk, pl, lk, tw, H, out_field, peak));                            \
   }
   switch (n) {
     DG_FOR_EACH_N(DG_CASE_N)
@@ -291,17 +309,25 @@ int nl_t(dg_handle *h, const CX *G, const CX *tw, int jmin, int jmax, const char
 
 }  // namespace
 
+int dg_cols_group(int n) {
+  ColPlan pl;
+  return cols_ra(n) || cols_plan(n, &pl) ? 1 << cols_log_kxg(n) : 0;
+}
+
 int dg_cols_inv(dg_handle *h, const double2 *const *f, int nf, int jmin, int jmax, long in_plane,
-                int rowlen, int n, int nk, const double2 *tw, double2 *H, long out_field) {
-  return inv_t(h, f, nf, jmin, jmax, in_plane, rowlen, n, nk, tw, H, out_field, "k_cols_inv");
+                int rowlen, int n, int nk, const double2 *tw, double2 *H, long out_field,
+                PeakOut peak) {
+  return inv_t(h, f, nf, jmin, jmax, in_plane, rowlen, n, nk, tw, H, out_field, peak, "k_cols_inv");
 }
 int dg_cols_inv(dg_handle *h, const double2 *const *f, int nf, int jmin, int jmax, long in_plane,
-                int rowlen, int n, int nk, const float2 *tw, float2 *H, long out_field) {
-  return inv_t(h, f, nf, jmin, jmax, in_plane, rowlen, n, nk, tw, H, out_field, "k_cols_inv_f32");
+                int rowlen, int n, int nk, const float2 *tw, float2 *H, long out_field,
+                PeakOut peak) {
+  return inv_t(h, f, nf, jmin, jmax, in_plane, rowlen, n, nk, tw, H, out_field, peak, "k_cols_inv_f32");
 }
 int dg_cols_inv(dg_handle *h, const float2 *const *f, int nf, int jmin, int jmax, long in_plane,
-                int rowlen, int n, int nk, const float2 *tw, float2 *H, long out_field) {
-  return inv_t(h, f, nf, jmin, jmax, in_plane, rowlen, n, nk, tw, H, out_field, "k_cols_inv_f32");
+                int rowlen, int n, int nk, const float2 *tw, float2 *H, long out_field,
+                PeakOut peak) {
+  return inv_t(h, f, nf, jmin, jmax, in_plane, rowlen, n, nk, tw, H, out_field, peak, "k_cols_inv_f32");
 }
 int dg_cols_fwd(dg_handle *h, const double2 *H, long in_field, int nf, int jmin, int jmax,
                 int rowlen, int n, int nk, const double2 *tw, double2 *const *f, long out_plane) {

@@ -41,7 +41,7 @@ template <int NT, typename CX, typename PA = CFieldPtrs, int PV = 0>
 __global__ void __launch_bounds__(NTHR) k_zinv(PA fields, int jmin, long ss, int nkxp,
                                               int NZr, int NKZ, FftPlan pl,
                                               const CX *__restrict__ tw,
-                                              CX *__restrict__ H, long Hfield) {
+                                              CX *__restrict__ H, long Hfield, PeakOut peak) {
   extern __shared__ double2 sm_raw[];
   CX *sm = reinterpret_cast<CX *>(sm_raw);
   const int NZ = NT ? NT : NZr;
@@ -90,9 +90,18 @@ __global__ void __launch_bounds__(NTHR) k_zinv(PA fields, int jmin, long ss, int
     res = fft_cta<NT, PV>(b0, b1, pl, KXG, sstr, stw, +1);
   }
   CX *out = H + f * Hfield + (long)j * NZ * nkxp;
+  unsigned pk = 0;
   for (int idx = tid; idx < KXG * NZ; idx += nthr) {
     const int c = idx % KXG, z = idx / KXG;
-    if (kx0 + c < nkxp) out[(long)z * nkxp + kx0 + c] = res[c * sstr + pad(z)];
+    if (kx0 + c >= nkxp) continue;
+    const CX v = res[c * sstr + pad(z)];
+    out[(long)z * nkxp + kx0 + c] = v;
+    if (!(peak.skip0 && kx0 + c == 0)) pk = max(pk, max(dg_mag(v.x), dg_mag(v.y)));
+  }
+  if (peak.p) {
+    pk = __reduce_max_sync(0xffffffffu, pk);
+    if ((tid & 31) == 0)
+      peak.p[(((long)f * peak.planes + j) * gridDim.x + blockIdx.x) * (NTHR / 32) + (tid >> 5)] = pk;
   }
 }
 
@@ -550,11 +559,12 @@ auto xc2r_cfl_kernel(int v) {
 template <typename CI, typename CX>
 static int cinv_t(dg_handle *h, const CI *const *fields, int nf, int jmin, int jmax,
                   long in_plane, int rowlen, int N, int NK, const FftPlan &pl, const CX *tw, CX *H,
-                  long out_field, bool plane_form = false) {
+                  long out_field, PeakOut peak, bool plane_form = false) {
   using PA = PtrArray<const CI>;
   if (jmax < jmin || nf <= 0) return DG_OK;
   if (!plane_form) {
-    const int s = dg_cols_inv(h, fields, nf, jmin, jmax, in_plane, rowlen, N, NK, tw, H, out_field);
+    const int s = dg_cols_inv(h, fields, nf, jmin, jmax, in_plane, rowlen, N, NK, tw, H, out_field,
+                              peak);
     if (s != 1) return s;
   }
   PA fp;
@@ -567,7 +577,7 @@ static int cinv_t(dg_handle *h, const CI *const *fields, int nf, int jmin, int j
     big_smem(kern);                                                                           \
     dg_kt_begin(h, "k_zinv", h->st);                                                          \
     DG_CUDA(dg_launch(h->pdl_zinv, kern, grid, dim3(NTHR), sm, h->st, fp, jmin, in_plane,     \
-                      rowlen, N, NK, pl, tw, H, out_field));                                  \
+                      rowlen, N, NK, pl, tw, H, out_field, peak));                            \
   }
   // compile-time lengths: the plane form's only (dg_cols_inv takes the others)
   if constexpr (std::is_same<CI, double2>::value && std::is_same<CX, double2>::value) {
@@ -585,20 +595,33 @@ static int cinv_t(dg_handle *h, const CI *const *fields, int nf, int jmin, int j
 
 int dg_cinv_g(dg_handle *h, const double2 *const *fields, int nf, int jmin, int jmax,
               long in_plane, int rowlen, int N, int NK, const FftPlan &pl, const double2 *tw,
-              double2 *H, long out_field) {
-  return cinv_t(h, fields, nf, jmin, jmax, in_plane, rowlen, N, NK, pl, tw, H, out_field);
+              double2 *H, long out_field, PeakOut peak) {
+  return cinv_t(h, fields, nf, jmin, jmax, in_plane, rowlen, N, NK, pl, tw, H, out_field, peak);
 }
 
 int dg_cinv_gf(dg_handle *h, const double2 *const *fields, int nf, int jmin, int jmax,
                long in_plane, int rowlen, int N, int NK, const FftPlan &pl, const float2 *tw,
-               float2 *H, long out_field) {
-  return cinv_t(h, fields, nf, jmin, jmax, in_plane, rowlen, N, NK, pl, tw, H, out_field);
+               float2 *H, long out_field, PeakOut peak) {
+  return cinv_t(h, fields, nf, jmin, jmax, in_plane, rowlen, N, NK, pl, tw, H, out_field, peak);
 }
 
 int dg_cinv_ff(dg_handle *h, const float2 *const *fields, int nf, int jmin, int jmax,
                long in_plane, int rowlen, int N, int NK, const FftPlan &pl, const float2 *tw,
-               float2 *H, long out_field) {
-  return cinv_t(h, fields, nf, jmin, jmax, in_plane, rowlen, N, NK, pl, tw, H, out_field);
+               float2 *H, long out_field, PeakOut peak) {
+  return cinv_t(h, fields, nf, jmin, jmax, in_plane, rowlen, N, NK, pl, tw, H, out_field, peak);
+}
+
+int dg_peak_len(int n, int rowlen) {
+  const int g = dg_cols_group(n);
+  return 4 * dg_cdiv(rowlen, g ? g : batch_for(n));  // a CTA of either kernel has four warps
+}
+
+PeakOut dg_peak_out(const dg_handle *h) {
+  PeakOut o;
+  o.p = h->peak;
+  o.planes = h->periodic ? h->NY : h->NY + 2;
+  o.skip0 = h->mixed && !h->periodic;
+  return o;
 }
 
 template <typename CX, typename PO, typename OUT>
@@ -650,9 +673,9 @@ int dg_cfwd_ff(dg_handle *h, const float2 *H, long in_field, int nf, int jmin, i
 static bool plane_lengths(const dg_handle *h);
 
 int dg_zinv(dg_handle *h, const double2 *const *fields, int nf, int jmin, int jmax, double2 *H,
-            bool plane_form) {
+            bool plane_form, PeakOut peak) {
   return cinv_t(h, fields, nf, jmin, jmax, h->ss, h->nkxp, h->NZ, h->NKZ, h->plz, h->twz, H,
-                (long)h->nplanes * h->NZ * h->nkxp, plane_form && plane_lengths(h));
+                (long)h->nplanes * h->NZ * h->nkxp, peak, plane_form && plane_lengths(h));
 }
 
 int dg_zfwd_planes(dg_handle *h, const double2 *H, int nf, int jmin, int jmax,

@@ -411,7 +411,7 @@ static int per_nonlinear_mixed(dg_handle *h, const PerConst &C) {
   const float2 *hy[3 + DG_MAX_TH];
   for (int f = 0; f < nf; f++) hy[f] = Hyf + f * hy_field(h);
   DG_TRY(dg_cinv_ff(h, hy, nf, 0, h->NY - 1, h->ss, h->nkxp, h->NZ, h->NKZ, h->plz, h->twz_f, Hf,
-                    h_field(h)));
+                    h_field(h), dg_peak_out(h)));
   if (!dg_per_rows_ok(h->NX, h->NTH)) {
     dg_set_error("mixed precision: no FP32 product kernel for this NX / N_TH");
     return DG_ERR_DIMS;
@@ -470,10 +470,11 @@ extern "C" int diablo_rk_per_1(dg_handle *h, int rk_step) {
                    hy_field(h)));
   const double2 *hy[3 + DG_MAX_TH];
   for (int f = 0; f < nf; f++) hy[f] = h->Hy + f * hy_field(h);
+  const bool rows = dg_per_rows_ok(h->NX, h->NTH);
   DG_TRY(dg_cinv_g(h, hy, nf, 0, h->NY - 1, h->ss, h->nkxp, h->NZ, h->NKZ, h->plz, h->twz, h->H,
-                   h_field(h)));
+                   h_field(h), rows ? dg_peak_out(h) : PeakOut()));
   // x rows: products
-  if (dg_per_rows_ok(h->NX, h->NTH)) {
+  if (rows) {
     DG_TRY(dg_per_rows(h));
   } else {
     // generic: physical fields, pointwise products, r2c of each product

@@ -24,6 +24,10 @@
 // work (32 x 8: 291 us at 256^3), except with two scalars, whose 5 x 16 points
 // spill in FP64 (256x64x64: 42 against 37 us).  At most 128 points FP64 fits three
 // CTAs per SM (128^3 with a scalar: 44 -> 40 us); above, that spills (228 -> 262).
+//
+// A scalar packed with U1, and the second scalar's product packed with the first's, are
+// scaled to one magnitude by a power of two before the transform and back after it
+// (dg_pair_shift; the largest of the planes of a warp's rows).
 #include "dg_internal.cuh"
 #include "fft_cols.cuh"
 
@@ -39,7 +43,8 @@ __host__ __device__ constexpr int pr_buf(int RF, int RS, int nth) {
 template <int RF, int RS, int NTH, typename CX>
 __global__ void __launch_bounds__(128, sizeof(CX) == 16 && RF * RS > 128 ? 2 : 3)
     k_per_rows(long nrows, const CX *__restrict__ H, long Hfield, const CX *__restrict__ tw,
-               CX *__restrict__ P, long Pfield) {
+               CX *__restrict__ P, long Pfield, int NZ, const unsigned *__restrict__ peak,
+               int planes, int plen) {
   using TR = typename CT<CX>::T;
   constexpr int NX = RF * RS, NKXP = NX / 3 + 1, RPW = 32 / RF;
   constexpr int NF = 3 + NTH, NPIN = (NF + 1) / 2, NPROD = 6 + 3 * NTH, NPP = (NPROD + 1) / 2;
@@ -58,26 +63,59 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 16 && RF * RS > 128 ? 2 : 3
   auto fa = [](int s) { return s < 2 ? s : 2 * s; };
   auto fb = [](int s) { return s == 0 ? 3 : s == 1 ? 2 : 2 * s + 1; };
   const CX *src = H + ro;
+  // a lane's share of the peaks of U1 and the scalars on its row's plane: on their way
+  // before the first bins, used behind them (96x64x96 in FP32 with a scalar: 14.7 us per
+  // launch; 16.8 with the shifts ahead of the bins' loads)
+  unsigned pk[1 + NTH];
+  if constexpr (NTH > 0) {
+    const unsigned row_c = (unsigned)(rr < nrows ? rr : nrows - 1);
+    const unsigned *p = peak + (long)(row_c / (unsigned)NZ) * plen;
+#pragma unroll
+    for (int i = 0; i <= NTH; i++) {
+      const unsigned *q = p + (long)(i ? 2 + i : 0) * planes * plen;
+      pk[i] = t < plen ? __ldg(q + t) : 0;
+#pragma unroll 1
+      for (int l = t + RF; l < plen; l += RF) pk[i] = max(pk[i], __ldg(q + l));
+    }
+  }
+  int d = 0, sh = 0;  // binary orders from TH1 to U1 and from TH2 to TH1
 #pragma unroll
   for (int i0 = 0; i0 < NPIN * RS; i0 += RF) {
     const int i = i0 + t, s = i / RS, b = i % RS;
-    if (on && i < NPIN * RS) {
+    const bool item = on && i < NPIN * RS;
+    CX ar[RF], cr[RF];
+    if (item) {
       const CX *ra = src + fa(s) * Hfield, *rb = src + fb(s) * Hfield;
       const bool two = fb(s) < NF;
-      CX v[RF];
 #pragma unroll
       for (int r = 0; r < RF; r++) {
         // bins NX/3 + 1 .. NX - NX/3 - 1 are zero
-        v[r] = CT<CX>::mk(0, 0);
+        ar[r] = cr[r] = CT<CX>::mk(0, 0);
         if (RS * r > KLO && RS * r + RS - 1 < KHI) continue;
         const int k = b + RS * r, kk = (k <= NX / 2) ? k : NX - k;
-        CX a = CT<CX>::mk(0, 0), c = CT<CX>::mk(0, 0);
         if (kk < NKXP) {
-          a = __ldg(ra + kk);
-          if (two) c = __ldg(rb + kk);
-          if (kk == 0) a.y = c.y = 0;
+          ar[r] = __ldg(ra + kk);
+          if (two) cr[r] = __ldg(rb + kk);
+          if (kk == 0) ar[r].y = cr[r].y = 0;
         }
-        v[r] = (k == kk) ? CT<CX>::mk(a.x - c.y, a.y + c.x) : CT<CX>::mk(a.x + c.y, c.x - a.y);
+      }
+    }
+    if (NTH > 0 && i0 == 0) {
+      int e[1 + NTH];
+#pragma unroll
+      for (int f = 0; f <= NTH; f++) e[f] = dg_mag_exp<TR>(__reduce_max_sync(0xffffffffu, pk[f]));
+      d = dg_pair_shift<TR>(e[0], e[NTH > 0], 1);
+      if constexpr (NTH == 2) sh = dg_pair_shift<TR>(e[1], e[2], 0);
+    }
+    if (item) {
+      const TR sc = dg_pow2<TR>(NTH > 0 && s == 0 ? d : 0);
+      CX v[RF];
+#pragma unroll
+      for (int r = 0; r < RF; r++) {
+        const CX a = ar[r], c = cr[r];
+        const int k = b + RS * r;
+        v[r] = (k <= NX / 2) ? CT<CX>::mk(a.x - sc * c.y, a.y + sc * c.x)
+                             : CT<CX>::mk(a.x + sc * c.y, sc * c.x - a.y);
       }
       dft<RF>(v, +1);
       CX *o = buf + s * SI + b;
@@ -102,7 +140,7 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 16 && RF * RS > 128 ? 2 : 3
 #pragma unroll
     for (int m = 0; m < RS; m++) {
       u[fa(s)][m] = v[m].x;
-      if (fb(s) < NF) u[fb(s)][m] = v[m].y;
+      if (fb(s) < NF) u[fb(s)][m] = NTH > 0 && s == 0 ? v[m].y * dg_pow2<TR>(-d) : v[m].y;
     }
   }
   __syncwarp();
@@ -121,7 +159,10 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 16 && RF * RS > 128 ? 2 : 3
       if (s0 + sl >= NPP) continue;
       CX v[RS];
 #pragma unroll
-      for (int m = 0; m < RS; m++) v[m] = CT<CX>::mk(prod(2 * (s0 + sl), m), prod(2 * (s0 + sl) + 1, m));
+      for (int m = 0; m < RS; m++) {
+        v[m] = CT<CX>::mk(prod(2 * (s0 + sl), m), prod(2 * (s0 + sl) + 1, m));
+        if (NTH == 2 && s0 + sl == 4) v[m].y *= dg_pow2<TR>(sh);  // (U3 TH1, U1 TH2)
+      }
       dft<RS>(v, -1);
 #pragma unroll
       for (int p = 0; p < RS; p++)
@@ -149,7 +190,11 @@ __global__ void __launch_bounds__(128, sizeof(CX) == 16 && RF * RS > 128 ? 2 : 3
       const CX zk = v[m];
       // A = (Z_k + conj Z_{N-k})/2, B = -i/2 (Z_k - conj Z_{N-k}), over NX
       o[k] = CT<CX>::mk(hx * (zk.x + zm.x), hx * (zk.y - zm.y));
-      if (two) o[Pfield + k] = CT<CX>::mk(hx * (zk.y + zm.y), -hx * (zk.x - zm.x));
+      TR hb = hx;
+      if constexpr (NTH == 2) {
+        if (s0 + sl == 4) hb *= dg_pow2<TR>(-sh);
+      }
+      if (two) o[Pfield + k] = CT<CX>::mk(hb * (zk.y + zm.y), -hb * (zk.x - zm.x));
     }
     __syncwarp();
   }
@@ -163,7 +208,7 @@ int pr_launch(dg_handle *h, const CX *H, const CX *tw, CX *P, const char *name) 
   constexpr int rows = 4 * (32 / RF);
   dg_kt_begin(h, name, h->st);
   kern<<<dg_cdiv(nrows, rows), 128, sizeof(CX) * rows * (size_t)pr_buf(RF, RS, NTH), h->st>>>(
-      nrows, H, pf, tw, P, pf);
+      nrows, H, pf, tw, P, pf, h->NZ, h->peak, h->NY, h->peak_len);
   DG_LAUNCHED();
   return DG_OK;
 }

@@ -202,6 +202,8 @@ extern "C" int64_t dg_state_bytes(const dg_params *p) {
   const int64_t planes = per ? nkyt : L;
   const int64_t ns = nkxp * nkzt * planes;
   int64_t b = 16 * ns * (3 * nf + 2);                      // cu, cf, rhs, cp, cr1
+  if (p->n_th > 0)                                        // peak
+    b += 4 * nf * (per ? p->ny : L) * dg_peak_len(p->nz, (int)nkxp);
   b += 8 * (3 * L + nkxp + nkzt + nkyt) + 16 * (p->nx + p->nz + p->ny) + 8 * 16 + 256;
   if (!per) {
     const int64_t hsz = planes * p->nz * nkxp;
@@ -375,6 +377,10 @@ extern "C" int diablo_gpu_init(const dg_params *p, const double *gy, void *strea
   DG_TRY(dalloc(h, &h->dmin_bits, 32));
   DG_TRY(dalloc(h, &h->dflag, 4));
   DG_CUDA(cudaMemsetAsync(h->dflag, 0, 4 * sizeof(int), h->st));
+  if (h->NTH > 0) {
+    h->peak_len = dg_peak_len(h->NZ, h->nkxp);
+    DG_TRY(dalloc(h, &h->peak, (size_t)h->nf * (h->periodic ? NY : L) * h->peak_len));
+  }
   const size_t ns = (size_t)h->nspec;
   for (int f = 0; f < h->nf; f++) {
     DG_TRY(dalloc(h, &h->cu[f], ns));
@@ -418,7 +424,7 @@ extern "C" int diablo_gpu_finalize(dg_handle *h) {
   cudaStreamSynchronize(h->st);
   cudaStreamSynchronize(h->st2);
   void *dp[] = {h->gyf, h->dy, h->dyf, h->kx, h->kz, h->ky, h->kx2, h->kz2, h->ky2, h->twx, h->twz,
-                h->twy, h->twx_f, h->twz_f, h->twy_f, h->dscal, h->cp, h->cr1, h->gphi, h->rem_a, h->rem_rb, h->cn_tab, h->cn_rows, h->rowc, h->col_dcase, h->col_dwork, h->H, h->G, h->work, h->dmin_bits, h->dflag, h->Hy, h->P,
+                h->twy, h->twx_f, h->twz_f, h->twy_f, h->dscal, h->cp, h->cr1, h->gphi, h->rem_a, h->rem_rb, h->cn_tab, h->cn_rows, h->rowc, h->col_dcase, h->col_dwork, h->H, h->G, h->work, h->dmin_bits, h->dflag, h->peak, h->Hy, h->P,
                 h->Q};
   for (void *q : dp) dg_free(h, q);
   dg_free(h, h->les_phys);
