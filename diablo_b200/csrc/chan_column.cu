@@ -266,7 +266,7 @@ template <int MT, int K, int FK, bool CPL, typename Table>
 __device__ __forceinline__ void col_rows(const FieldCoef &k, bool old_cf, int L, long ss, long mg,
                                          int j0, int nr, int nseg, bool mean, double Kh, double kk,
                                          int wlo,
-                                         const double2 *__restrict__ cu, const double2 *nl,
+                                         const double2 *cu, const double2 *nl,
                                          double2 *cff, const double2 *__restrict__ cpp,
                                          double2 *dst, const double *TB, const double *RC, int LP,
                                          double2 *TG, double *TP, Table table) {
@@ -275,7 +275,10 @@ __device__ __forceinline__ void col_rows(const FieldCoef &k, bool old_cf, int L,
   const long o0 = (long)j0 * ss + mg;
   auto in = [&](int q) { return q < nr && j0 + q >= k.lo && j0 + q <= k.hi; };
   // ---- 1. R.  Every input row is on its way before the first is used, and
-  // before the wait for the table rows.
+  // before the wait for the table rows.  A scalar written in place has dst == cu, and the
+  // rows j0-1 and j0+K are other threads': plain loads there (the read-only path and
+  // restrict want data that the launch does not write), all of them before the
+  // first barrier of carry(), and every store to dst after its second.
   double2 r[K], p[K + 1], u[K + 2], v[K];  // CF_old, CP rows j0-1 .., CU rows j0-1 .., NL
 #pragma unroll
   for (int q = 0; q < K; q++) r[q] = (old_cf && in(q)) ? cff[o0 + q * ss] : z2();
@@ -287,7 +290,9 @@ __device__ __forceinline__ void col_rows(const FieldCoef &k, bool old_cf, int L,
 #pragma unroll
   for (int q = 0; q < K + 2; q++) {
     const int j = j0 + q - 1;
-    u[q] = (nr > 0 && j >= 0 && j < L) ? __ldg(cu + o0 + (q - 1) * ss) : z2();
+    const bool have = nr > 0 && j >= 0 && j < L;
+    if constexpr (FK == 2) u[q] = have ? cu[o0 + (q - 1) * ss] : z2();
+    else u[q] = have ? __ldg(cu + o0 + (q - 1) * ss) : z2();
   }
 #pragma unroll
   for (int q = 0; q < K; q++) v[q] = in(q) ? nl[o0 + q * ss] : z2();

@@ -605,3 +605,31 @@ def test_register_rows_factor_5_and_9_match_oracle(nx, n_th, ny, nz, chunk):
         ch.step(s)
     compare(ref, ch, fields(p))
     ch.close()
+
+
+@pytest.mark.parametrize("case", ["coupled", "uncoupled"])
+@pytest.mark.parametrize("ny,mt", [(46, 4), (47, 2), (47, 16), (65, 2), (98, 8), (131, 4), (131, 16),
+                                   (150, 16)])
+def test_column_stage_tall_columns_match_oracle(case, ny, mt):
+    """The column stage with 5 rows per segment (NY + 2 > 48; 46 is the tallest with 3), many
+    quads of segments and partial last ones, against the oracle.  "uncoupled": a scalar written
+    in place, whose segments read rows that their neighbours overwrite; "coupled": every
+    field's right-hand side reads others (rotation, gravity in three directions, DRHODX/Z)."""
+    p, gy = configs.kh_shear_layer(nx=16, ny=ny, nz=16)
+    p = p.replace(variable_dt=1, update_dt=1, cfl=0.4, n_th=2)
+    p.pr = [1.0, 0.7, 1, 1]
+    p.th_bc_ymin, p.th_bc_ymax = [0, 1, 0, 0], [0, 1, 0, 0]
+    p.th_bc_ymin_c1, p.th_bc_ymax_c1 = [-1.0, 0.1, 0, 0], [1.0, -0.2, 0, 0]
+    if case == "coupled":
+        p = p.replace(i_ro=0.3, grav_x=0.2, grav_z=-0.1)
+        p.ri = [0.1, 0.05, 0, 0]
+        p.drhodx, p.drhodz = [0.0, 0.3, 0, 0], [0.0, -0.2, 0, 0]
+    else:
+        p.ri = [0.0, 0.0, 0, 0]
+    ref, ch, _ = start_pair(p, gy, ics.kh_shear_layer, seed=21)
+    ch.tune_set(cn_mt=mt)
+    for s in range(1, 6):
+        ref.step(s)
+        ch.step(s)
+    compare(ref, ch, fields(p) + ["CP"], tol=1e-10)
+    ch.close()
