@@ -80,21 +80,34 @@ std::string shape_key(const dg_params &p) {
   return b;
 }
 
-}  // namespace
-
-int dg_default_col_mt(const dg_handle *h) {
-  // enough CTAs for about three per SM
+// enough CTAs for about three per SM; ss: retained modes per plane
+int default_col_mt(long ss) {
   for (int mt : {16, 8})
-    if ((h->ss + mt - 1) / mt >= 3 * 148) return mt;
+    if ((ss + mt - 1) / mt >= 3 * 148) return mt;
   return 4;
 }
 
 // 8 modes fill whole 128-byte lines of a row (40.8 us per launch at
 // Re_tau = 180, 44.4 with 4, 44 with 16; 1107 us at 512x257x384, 1151 with 4);
 // 4 where 8 would leave SMs without a CTA
-int dg_default_cn_mt(const dg_handle *h) {
-  return (long)h->nf * ((h->ss + 7) / 8) < 148 ? 4 : 8;
+int default_cn_mt(int nf, long ss) { return nf * ((ss + 7) / 8) < 148 ? 4 : 8; }
+
+// what a handle of the shape starts with
+TuneRec shape_defaults(const std::string &key) {
+  int nx = 0, ny = 0, nz = 0, nth = 0;
+  TuneRec rec = {{8, 0, 0, 8, 1, 0}};  // no shape_key: no handle looks it up
+  if (sscanf(key.c_str(), "%dx%dx%d_th%d_", &nx, &ny, &nz, &nth) == 4) {
+    const long ss = (long)(nx / 3 + 1) * (2 * (nz / 3) + 1);
+    rec.v[0] = default_col_mt(ss);
+    rec.v[3] = default_cn_mt(3 + nth, ss);
+  }
+  return rec;
 }
+
+}  // namespace
+
+int dg_default_col_mt(const dg_handle *h) { return default_col_mt(h->ss); }
+int dg_default_cn_mt(const dg_handle *h) { return default_cn_mt(h->nf, h->ss); }
 
 static void invalidate_graphs(dg_handle *h) {
   dg_graphs_free(h);
@@ -345,8 +358,8 @@ extern "C" int dg_tune_cache_save(const char *path) {
 
 // Reads the file dg_tune_cache_save writes (a JSON object of objects whose
 // values are integers) and merges its entries into the table.  Unknown
-// tunable names are ignored; an entry lacking one keeps that tunable's
-// default; anything that is not this shape of JSON is an error and leaves
+// tunable names are ignored; an entry lacking one gets the default of its
+// shape for it; anything that is not this shape of JSON is an error and leaves
 // the table as it was.
 extern "C" int dg_tune_cache_load(const char *path) {
   if (!path) return DG_ERR_ARG;
@@ -391,7 +404,7 @@ extern "C" int dg_tune_cache_load(const char *path) {
     do {
       std::string key;
       if (!str(key) || !ch(':') || !ch('{')) return bad();
-      TuneRec rec = {{8, 0, 0, 4, 1, 0}};
+      TuneRec rec = shape_defaults(key);
       if (!ch('}')) {
         do {
           std::string name;

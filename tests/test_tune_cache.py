@@ -37,3 +37,19 @@ def test_cache_rejects_malformed_file(tmp_path):
     with pytest.raises(_lib.DiabloError):
         _lib.tune_cache_load(str(bad))
     assert _lib.tune_cache_get(p, 3) == 8          # the table is as it was
+
+
+@pytest.mark.parametrize("shape,col,cn", [((128, 129, 128), 8, 8), ((16, 17, 16), 4, 4),
+                                          ((256, 33, 256), 16, 8), ((64, 33, 16), 4, 4)])
+def test_missing_tunables_get_the_defaults_of_the_shape(tmp_path, shape, col, cn):
+    """The modes per CTA depend on the shape: enough CTAs for three per SM of 148 (REM_DIV), 4
+    where 8 leave SMs without a CTA (Crank-Nicolson: 3 fields of (nx/3+1)(2(nz/3)+1) modes)."""
+    nx, ny, nz = shape
+    p, _ = configs.channel_re180(nx=nx, ny=ny, nz=nz)
+    key = f"{nx}x{ny}x{nz}_th0_fp64"
+    src = tmp_path / "in.json"
+    src.write_text(json.dumps({key: {"xrow_chunk": 4}}))
+    _lib.tune_cache_load(str(src))
+    assert _lib.tune_cache_get(p, 1) == 4
+    assert _lib.tune_cache_get(p, 0) == col
+    assert _lib.tune_cache_get(p, 3) == cn
