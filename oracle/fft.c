@@ -20,9 +20,8 @@
 #include <string.h>
 #include "oracle_int.h"
 
-#define MAX_PLANS 64  /* transform lengths of one process */
-
-typedef struct {
+typedef struct plan {
+  struct plan *next;
   int n;
   int nfac;
   int fac[64];            /* pairs (p, m) per recursion level */
@@ -30,20 +29,24 @@ typedef struct {
   cplx *tw_inv;           /* exp(+2 pi i k / n) */
 } plan_t;
 
-static plan_t plans[MAX_PLANS];
-static int nplans = 0;
+/* every length's plan, newest first; a plan is complete before it is linked and
+   stays for the process, so readers need no lock */
+static plan_t *plans = NULL;
+
+static plan_t *find_plan(int n) {
+  plan_t *pl = __atomic_load_n(&plans, __ATOMIC_ACQUIRE);
+  while (pl && pl->n != n) pl = pl->next;
+  return pl;
+}
 
 static const plan_t *get_plan(int n) {
-  for (int i = 0; i < nplans; i++)
-    if (plans[i].n == n) return &plans[i];
-  plan_t *pl;
+  plan_t *pl = find_plan(n);
+  if (pl) return pl;
 #pragma omp critical(orc_fft_plan)
   {
-    pl = NULL;
-    for (int i = 0; i < nplans; i++)
-      if (plans[i].n == n) pl = &plans[i];
+    pl = find_plan(n);
     if (!pl) {
-      pl = &plans[nplans];
+      pl = (plan_t *)calloc(1, sizeof(plan_t));
       pl->n = n;
       pl->tw_fwd = (cplx *)malloc(sizeof(cplx) * n);
       pl->tw_inv = (cplx *)malloc(sizeof(cplx) * n);
@@ -72,8 +75,8 @@ static const plan_t *get_plan(int n) {
         nf++;
       }
       pl->nfac = nf;
-      __sync_synchronize();
-      nplans++;
+      pl->next = plans;
+      __atomic_store_n(&plans, pl, __ATOMIC_RELEASE);
     }
   }
   return pl;

@@ -8,6 +8,9 @@ RK3/CN scheme (a decaying Fourier mode; the laminar Poiseuille profile), and
 the reference's own KH grid fixture (tests/test_inputs.py).
 """
 import math
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -177,3 +180,20 @@ def test_host_spectral_ic_matches_oracle_transform():
     phys = rng.standard_normal(p.phys_shape())
     np.testing.assert_allclose(ics.to_spectral_chan(phys, p), o.to_fourier(phys), rtol=0,
                                atol=1e-15)
+
+
+def test_fft_plans_of_many_lengths():
+    """More transform lengths in one process than a fixed table would hold: every one, the
+    earlier ones again, from a process of its own (an overflow corrupts memory)."""
+    code = """
+import numpy as np, oracle as O
+rng = np.random.default_rng(1)
+for again in range(2):
+    for n in range(2, 302, 2):
+        x = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+        assert np.abs(O.fft1d(x, -1) - np.fft.fft(x)).max() <= 1e-12 * n, n
+print("all lengths")
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.abspath(O.__file__)))
+    assert r.returncode == 0 and "all lengths" in r.stdout, (r.returncode, r.stderr[-500:])
