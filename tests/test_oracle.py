@@ -188,12 +188,15 @@ def test_fft_plans_of_many_lengths():
     code = """
 import numpy as np, oracle as O
 rng = np.random.default_rng(1)
+lengths = sorted(2 ** a * 3 ** b * 5 ** c for a in range(1, 9) for b in range(4) for c in range(4))
 for again in range(2):
-    for n in range(2, 302, 2):
+    for n in lengths:  # 128 of them
         x = rng.standard_normal(n) + 1j * rng.standard_normal(n)
         assert np.abs(O.fft1d(x, -1) - np.fft.fft(x)).max() <= 1e-12 * n, n
 print("all lengths")
 """
+    here = os.path.dirname(os.path.abspath(O.__file__))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([here, os.path.dirname(here)]))
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
-                       cwd=os.path.dirname(os.path.abspath(O.__file__)))
+                       env=env)
     assert r.returncode == 0 and "all lengths" in r.stdout, (r.returncode, r.stderr[-500:])
