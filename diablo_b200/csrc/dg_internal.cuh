@@ -182,7 +182,7 @@ int dg_default_col_mt(const dg_handle *h);
 int dg_default_cn_mt(const dg_handle *h);
 bool dg_mixed_ok(int nx, int nz, int n_th);
 bool dg_per_mixed_ok(int nx, int n_th);
-bool dg_per_rows_ok(int nx, int n_th);  // per_rows.cu
+bool dg_per_rows_ok(int nx, int n_th, bool mixed);  // per_rows.cu
 int dg_per_rows(dg_handle *h);
 
 void dg_graphs_free(dg_handle *h);

@@ -372,7 +372,7 @@ int dg_per_init(dg_handle *h) {
   DG_TRY(al(&h->Q, (size_t)np * fy_field(h)));         // Fy
   // physical scratch: 6 fields for POISSON_P_PER; the generic product path
   // (lengths or scalar counts that k_per_rows does not take) needs nf + np
-  const int nphys = dg_per_rows_ok(h->NX, h->NTH) ? 6 : (h->nf + np > 6 ? h->nf + np : 6);
+  const int nphys = dg_per_rows_ok(h->NX, h->NTH, h->mixed) ? 6 : (h->nf + np > 6 ? h->nf + np : 6);
   h->work_bytes = sizeof(double) * (size_t)phys_field(h) * nphys;
   if (h->work_bytes < sizeof(double) * 8 * (size_t)h->nkyt)
     h->work_bytes = sizeof(double) * 8 * (size_t)h->nkyt;
@@ -412,7 +412,7 @@ static int per_nonlinear_mixed(dg_handle *h, const PerConst &C) {
   for (int f = 0; f < nf; f++) hy[f] = Hyf + f * hy_field(h);
   DG_TRY(dg_cinv_ff(h, hy, nf, 0, h->NY - 1, h->ss, h->nkxp, h->NZ, h->NKZ, h->plz, h->twz_f, Hf,
                     h_field(h), dg_peak_out(h)));
-  if (!dg_per_rows_ok(h->NX, h->NTH)) {
+  if (!dg_per_rows_ok(h->NX, h->NTH, h->mixed)) {
     dg_set_error("mixed precision: no FP32 product kernel for this NX / N_TH");
     return DG_ERR_DIMS;
   }
@@ -470,7 +470,7 @@ extern "C" int diablo_rk_per_1(dg_handle *h, int rk_step) {
                    hy_field(h)));
   const double2 *hy[3 + DG_MAX_TH];
   for (int f = 0; f < nf; f++) hy[f] = h->Hy + f * hy_field(h);
-  const bool rows = dg_per_rows_ok(h->NX, h->NTH);
+  const bool rows = dg_per_rows_ok(h->NX, h->NTH, h->mixed);
   DG_TRY(dg_cinv_g(h, hy, nf, 0, h->NY - 1, h->ss, h->nkxp, h->NZ, h->NKZ, h->plz, h->twz, h->H,
                    h_field(h), rows ? dg_peak_out(h) : PeakOut()));
   // x rows: products

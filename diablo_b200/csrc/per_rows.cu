@@ -223,8 +223,10 @@ int pr_th(dg_handle *h, const CX *H, const CX *tw, CX *P, const char *name) {
 
 }  // namespace
 
-// lengths of the FP32 form (dg_per_mixed_ok), and those of FP64 only
-bool dg_per_rows_ok(int nx, int nth) {
+// what dg_per_rows has an instance for: in FP32 the lengths that dg_per_mixed_ok admits,
+// in FP64 further ones
+bool dg_per_rows_ok(int nx, int nth, bool mixed) {
+  if (mixed) return dg_per_mixed_ok(nx, nth);
   if (nth > 2) return false;
   switch (nx) {
     case 16: case 32: case 48: case 64: case 96: case 128: case 256: case 20: case 24: case 30:
