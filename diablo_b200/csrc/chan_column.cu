@@ -49,6 +49,7 @@
 // The same kernel serves one case (a one-case table) and the ensemble
 // server's groups (a ragged work list over every member), so a case
 // computes with the same machine code either way.
+#include <stdio.h>
 #include <string.h>
 
 #include <algorithm>
@@ -597,7 +598,10 @@ static int col_mt(const dg_handle *h, int want) {
 
 static int col_fits(const dg_handle *h, int mt) {
   if (dg_col_smem(h, mt) > 220 * 1024 || col_threads(h, mt) > COL_MAX_THR) {
-    dg_set_error("column kernel: NY too large for two modes per CTA (NY + 2 <= 1024)");
+    char b[96];
+    snprintf(b, sizeof(b), "column kernel: NY too large for two modes per CTA (NY + 2 <= %d)",
+             COL_MAX_THR / 2 * SEG_K);
+    dg_set_error(b);
     return DG_ERR_DIMS;
   }
   return DG_OK;

@@ -633,3 +633,13 @@ def test_column_stage_tall_columns_match_oracle(case, ny, mt):
         ch.step(s)
     compare(ref, ch, fields(p) + ["CP"], tol=1e-10)
     ch.close()
+
+
+def test_column_height_limit_is_the_one_reported():
+    """A column that does not fit the column kernel is refused with the true limit: 512 threads
+    per CTA, two modes, 5 rows per segment."""
+    p, gy = configs.channel_re180(nx=16, ny=1300, nz=16)
+    ch = channel(p, gy)
+    with pytest.raises(Exception, match=r"NY \+ 2 <= 1280"):
+        ch.rk_chan_1(1, 1)
+    ch.close()
