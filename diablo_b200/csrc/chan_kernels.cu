@@ -8,8 +8,10 @@
 //   k_xrows     per physical z-row, marching up in y: x c2r of every field,
 //               all products/fluxes of for/channel.f:409-571,665-720, x r2c,
 //               and the combination into 2 arrays per field
-//               (A: to be multiplied by -i kz, B: the rest); chan_xrows.cu for rows of
-//               16 to 128 points, k_xmarch (chan_xmarch.cu) for 192 to 512.  Other row
+//               (A: to be multiplied by -i kz, B: the rest).  chan_xrows.cu and
+//               chan_xrows64.cu list the row lengths (16 to 128 points, in FP64
+//               others up to 320); k_xmarch (chan_xmarch.cu) runs 384 and 512, 256
+//               (in FP64 with scalars) and in FP32 192.  Other row
 //               lengths and N_TH > 2 take two launches instead: k_xc2r of
 //               every plane into physical space, then k_xprod (products, x
 //               r2c and the combination, one product pair per CTA).

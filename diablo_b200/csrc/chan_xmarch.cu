@@ -20,7 +20,7 @@
 // pass; the physical rows never reach HBM.  What bounds it is shared-memory
 // bandwidth: about 350 KB of it per row and plane at NX = 512 with a scalar.
 //
-// At 512x257x384 with a scalar it takes 2.08 ms per launch in FP64 (1.38 in
+// At 512x257x384 with a scalar it takes 2.12 ms per launch in FP64 (1.43 in
 // FP32), where a c2r launch into an array of physical rows and a launch per
 // product pair took 1.20 + 3.39 ms (0.60 + 3.63); 0.21 ms at 192x193x192 in FP32
 // (0.06 + 0.38).  ncu at 512x65x384: shared memory busy 47% of the time, 12
@@ -52,7 +52,7 @@ __host__ __device__ constexpr int xm_sstr(int T, int R1, int esz) {
   const int w = esz == 16 ? 8 : 16;
   // (8-byte values: a half warp of the passes with T/R = 8 covers two
   // sub-transforms, whose buffers then must lie 8 values apart)
-  const int want = esz == 16 ? (R1 == 2 ? 4 : R1 == 3 ? 3 : R1 == 4 ? 2 : R1 == 5 ? 5 : 1) : 8;
+  const int want = esz == 16 ? (R1 == 3 ? 3 : 2) : 8;  // R1 is 3 or 4
   int s = T + (T - 1) / 16;
   while (s % w != want) s++;
   return s;

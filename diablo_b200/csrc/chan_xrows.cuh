@@ -18,7 +18,7 @@
 // passes, output) made 6 each; that bandwidth bounded the stage (60% of its
 // peak), which one warp per row with Stockham passes took 73 us for at
 // 128x129x128 and now takes 55 (events around eager launches): 29 -> 17 us at 128x65x32
-// with a scalar, 79 -> 31 at 96x65x96, 75 -> 45 at 64x129x128 with two; FP32
+// with a scalar, 79 -> 31 at 96x65x96, 75 -> 47 at 64x129x128 with two; FP32
 // 59 -> 49 at 128x129x128.  Two CTAs per SM at up to 255 registers: a lane's points of two
 // planes and its RF values are registers (with 168 and spills 60 us; FP32
 // without scalars fits 168 and three CTAs, 49 us against 55).
@@ -27,7 +27,8 @@
 // signals go through in batches of NB = RF / RS, one item per lane.  Members that
 // have different units are brought to one magnitude by a power of two before a transform
 // and back after it (dg_pair_shift): a scalar packed with U1, the second scalar
-// packed with the first.
+// packed with the first (0 to 6% per launch with scalars: 30.4 -> 30.8 us at 96x65x96
+// with one, 124 -> 132 at 320x65x48 with two).
 #pragma once
 
 #include <math.h>

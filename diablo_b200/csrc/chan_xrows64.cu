@@ -1,7 +1,7 @@
 // k_xrows (chan_xrows.cuh) in FP64 for further lengths with factors 2, 3 and 5: the
 // rule, the dispatch and the shortest ones.  They replaced a c2r launch and a
-// launch per product pair with run-time transform plans (per launch, a scalar: 60x33x30 30 -> 14 us,
-// 150x65x48 101 -> 33, 72x74x324 261 -> 74, 240x65x48 147 -> 51; 320x65x48 with two 196 -> 130).
+// launch per product pair with run-time transform plans (per launch, a scalar: 60x33x30 30 -> 16 us,
+// 150x65x48 101 -> 34, 72x74x324 261 -> 76, 240x65x48 147 -> 53; 320x65x48 with two 196 -> 132).
 #include "chan_xrows.cuh"
 
 int dg_xrows64_l(dg_handle *h, int ja, int jb);

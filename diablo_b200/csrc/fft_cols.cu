@@ -125,13 +125,10 @@ __global__ void __launch_bounds__(COLS_THR, 4)
 
 // The channel's z forward: both product arrays of a field, A and B, on one
 // plane, and the nonlinear term -i kz A + B of every retained mode.  A goes
-// first; its outputs, times -i kz, stay in the slots of shared memory they came
-// from until B's are there.
+// first; its outputs stay in the slots of shared memory they came from until
+// B's are there (StoreNl takes them times -i kz).
 template <typename CX>
 struct KeepA {
-  const double *kz;
-  int n, nk;
-  double rn;
   template <int R>
   __device__ __forceinline__ void put(CX *v, int o, int step, int, CX *p, int lk) const {
 #pragma unroll
@@ -198,7 +195,7 @@ __global__ void __launch_bounds__(COLS_THR, 4)
   cols_front<NT, -1, LK>(sb, pl, lk, tw, LoadBins<CX>{ga + gfield, rowlen, ncol});
   // each thread keeps A's outputs in the slots it reads them from, and takes
   // the same items again for B: no barrier between
-  cols_back<NT, -1, LK>(sa, pl, lk, KeepA<CX>{kz, n, nk, rn});
+  cols_back<NT, -1, LK>(sa, pl, lk, KeepA<CX>{});
   cols_back<NT, -1, LK>(sb, pl, lk,
                     StoreNl<CX>{rhs(f) + (long)j * out_plane + c0, sa, sb, kz, n, nk, rowlen, ncol,
                                 rn});

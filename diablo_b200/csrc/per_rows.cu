@@ -14,15 +14,15 @@
 // Measured per launch, from one warp per row with those passes: FP64 256^3 368 ->
 // 225 us (6 arrays of 86 x 256^2 bins written, 3 read: 812 MB at 3.6 TB/s; with 255
 // registers 8 warps share an SM, and the latency of loads and FP64 bounds it), with a
-// scalar 256x64x128 81 -> 50, 128^3 53 -> 31, 32^3 8.6 -> 7.4; FP32 128^3 33 -> 23,
+// scalar 256x64x128 81 -> 52, 128^3 53 -> 31, 32^3 8.6 -> 7.4; FP32 128^3 33 -> 23,
 // 96x64x96 with a scalar 25 -> 15.  The lengths with a factor 5 or 9, FP64 only, took
 // a c2r launch per field, the products through physical arrays and an r2c launch
-// per product: 192x64x64 with a scalar 204 -> 25 us, 100x64x64 156 -> 17.
+// per product: 192x64x64 with a scalar 204 -> 27 us, 100x64x64 156 -> 17.
 //
 // RS is 8 or more where the row is long, so that a lane's forward step feeds full
 // registers; 16 x 16 at 256 points keeps every lane of the inverse's radix-16 step at
 // work (32 x 8: 291 us at 256^3), except with two scalars, whose 5 x 16 points
-// spill in FP64 (256x64x64: 42 against 37 us).  At most 128 points FP64 fits three
+// spill in FP64 (256x64x64: 42 against 37 us before the shifts below).  At most 128 points FP64 fits three
 // CTAs per SM (128^3 with a scalar: 44 -> 40 us); above, that spills (228 -> 262).
 //
 // A scalar packed with U1, and the second scalar's product packed with the first's, are

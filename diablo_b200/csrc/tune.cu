@@ -16,9 +16,10 @@
 //                       chunks keep the intermediate planes in L2.
 //   DG_TUNE_PDL         1 (default): the substep kernels are launched with
 //                       programmatic dependent launch; 0: plain launches.
-//   DG_TUNE_FFT_PLAN    radix order of the x and z transform plans: 0 the
-//                       largest radix first (128 = 16 x 8), 1 the reverse
-//                       (128 = 8 x 16).  Same transform, different shared-
+//   DG_TUNE_FFT_PLAN    radix order of the transforms that run as passes in
+//                       shared memory (the z forward with LES, COURANT's x
+//                       transform): 0 the largest radix first (128 = 16 x 8), 1 the
+//                       reverse (128 = 8 x 16).  Same transform, different shared-
 //                       memory strides, twiddle reuse and registers; lengths
 //                       whose factors are all equal have one plan.
 //   DG_TUNE_PLANE_XZ    1 (default): the LES model's transforms between

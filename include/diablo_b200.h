@@ -317,7 +317,8 @@ int dg_server_query(dg_server *s, dg_server_stats *st);
 /* Server options, set before the first dg_server_submit.
  * DG_SERVER_GROUP_CASES = G > 0: cases of similar size step together in
  * groups of up to G, one CUDA graph per group step, with one ragged column
- * launch per substep covering every member's (case, mode tile) work list;
+ * launch per substep covering every member's (case, mode tile) work list (so
+ * members also share the column kernel's modes per CTA and rows per segment);
  * 0 (default): every case steps on its own.  Results are the same either
  * way.  LES cases and cases with COURANT at an UPDATE_DT other than 1 always
  * step on their own. */
