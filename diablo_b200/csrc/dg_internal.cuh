@@ -353,11 +353,14 @@ __device__ __forceinline__ int dg_peak_exp(const unsigned *__restrict__ p, int l
 }
 // d for members with the biased exponents ea and eb: the second `below` binary orders
 // under the first.  One for a scalar with U1, whose error all fields see (U2's is
-// 1.01 times what it is beside a small scalar, 1.05 with none).  No shift where a member
-// is all zeros (or denormal) or not finite; the limit keeps 2^d and what it scales in range.
+// 1.01 times what it is beside a small scalar, 1.05 with none).  A member that is all
+// zeros (or denormal) is taken for that much smaller than the limit: a scalar without
+// fluctuations keeps none of U1's rounding.  No shift where one is not finite; the limit
+// keeps 2^d and what it scales in range.
 template <typename T> __device__ __forceinline__ int dg_pair_shift(int ea, int eb, int below) {
   constexpr int TOP = sizeof(T) == 4 ? 255 : 2047, LIM = sizeof(T) == 4 ? 60 : 500;
-  if (ea == 0 || eb == 0 || ea == TOP || eb == TOP) return 0;
+  if (ea == TOP || eb == TOP) return 0;
+  if (ea == 0 || eb == 0) return ea == eb ? 0 : eb == 0 ? LIM : -LIM;
   return max(-LIM, min(LIM, ea - eb - below));
 }
 template <typename T> __device__ __forceinline__ T dg_pow2(int d) {
