@@ -200,7 +200,7 @@ void dg_kt_free(dg_handle *h);
 // common kernel-launch helpers (defined in fft_kernels.cu)
 // Where an inverse column transform leaves the largest component of what it writes
 // per field and plane, one value per warp: the bits of its absolute value (double:
-// the high word).  The row kernels take the power of two from it that brings two
+// the high word); for U1 and the scalars, fields 0 and 3...  The row kernels take the power of two from it that brings two
 // packed fields to one magnitude (dg_pair_shift).  null: not wanted.
 struct PeakOut {
   unsigned *p = nullptr;  // [nf][planes][dg_peak_len]
@@ -340,16 +340,10 @@ __device__ __forceinline__ unsigned dg_mag(double x) { return __double2hiint(x) 
 template <typename T> __device__ __forceinline__ int dg_mag_exp(unsigned m) {
   return (int)(m >> (sizeof(T) == 4 ? 23 : 20));
 }
-// biased exponent of the largest of a field's len values of one plane
-template <typename T>
-__device__ __forceinline__ int dg_peak_exp(const unsigned *__restrict__ p, int len) {
-  unsigned m = 0;
-#pragma unroll 4
-  for (int i = 0; i < len; i += 4) {  // len is a multiple of 4, and so are the planes' offsets
-    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p + i));
-    m = max(max(m, max(v.x, v.y)), max(v.z, v.w));
-  }
-  return dg_mag_exp<T>(m);
+// the larger of m and 4 PeakOut values
+__device__ __forceinline__ unsigned dg_peak4(const unsigned *__restrict__ p, unsigned m) {
+  const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p));
+  return max(max(m, max(v.x, v.y)), max(v.z, v.w));
 }
 // d for members with the biased exponents ea and eb: the second `below` binary orders
 // under the first.  One for a scalar with U1, whose error all fields see (U2's is
@@ -379,10 +373,17 @@ __device__ __forceinline__ void dg_plane_shifts(int *sh, const unsigned *__restr
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const unsigned *p = peak + (long)(pl0 + i) * len;
     const long fs = (long)planes * len;
-    const int e0 = dg_peak_exp<T>(p, len), e1 = dg_peak_exp<T>(p + 3 * fs, len);
+    unsigned m0 = 0, m1 = 0, m2 = 0;
+#pragma unroll 4
+    for (int l = 0; l < len; l += 4) {  // len is a multiple of 4, and so are the planes' offsets
+      m0 = dg_peak4(p + l, m0);
+      m1 = dg_peak4(p + 3 * fs + l, m1);
+      if constexpr (NTH == 2) m2 = dg_peak4(p + 4 * fs + l, m2);
+    }
+    const int e0 = dg_mag_exp<T>(m0), e1 = dg_mag_exp<T>(m1);
     int hi = 0;
     if constexpr (NTH == 2) {
-      const int e2 = dg_peak_exp<T>(p + 4 * fs, len);
+      const int e2 = dg_mag_exp<T>(m2);
       hi = sizeof(T) == 4 ? e1 << 8 | e2 : dg_pair_shift<T>(e1, e2, 0);
     }
     sh[i] = (hi << 16) | (dg_pair_shift<T>(e0, e1, 1) & 0xffff);

@@ -40,7 +40,7 @@ struct LoadBins {
   }
 };
 
-// PK: *pk becomes the largest component's magnitude of the columns but cskip
+// PK, and pk given: *pk becomes the largest component's magnitude of the columns but cskip
 template <typename CX, bool PK>
 struct StoreBins {
   CX *out;
@@ -52,7 +52,7 @@ struct StoreBins {
     if (c >= ncol) return;
 #pragma unroll
     for (int m = 0; m < R; m++) out[(long)(o + m * step) * rowlen + c] = v[m];
-    if constexpr (PK) {
+    if (PK && pk) {
       unsigned t = 0;
 #pragma unroll
       for (int m = 0; m < R; m++) t = max(t, max(dg_mag(v[m].x), dg_mag(v[m].y)));
@@ -95,10 +95,11 @@ __global__ void __launch_bounds__(COLS_THR, 4)
   cols_front<NT, +1>(sm, pl, lk, tw,
                      LoadModes<CI, CX>{fields(f) + (long)j * in_plane + c0, n, nk, rowlen, ncol});
   unsigned pk = 0;
+  const bool want = PK && (f == 0 || f >= 3);  // U1 and the scalars
   cols_back<NT, +1>(sm, pl, lk,
                     StoreBins<CX, PK>{H + f * out_field + (long)j * n * rowlen + c0, rowlen, ncol,
-                                      &pk, peak.skip0 && c0 == 0 ? 0 : -1});
-  if constexpr (PK) {
+                                      want ? &pk : nullptr, peak.skip0 && c0 == 0 ? 0 : -1});
+  if (PK && want) {
     pk = __reduce_max_sync(0xffffffffu, pk);
     if ((threadIdx.x & 31) == 0)
       peak.p[(((long)f * peak.planes + j) * gridDim.x + blockIdx.x) * (COLS_THR / 32) +
